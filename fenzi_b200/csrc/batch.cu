@@ -485,7 +485,7 @@ struct Job {
 };
 
 // Device bytes of one uploaded system, an upper estimate of build_engine's allocations:
-// ~140 B per atom of atom, slot and PME-binning arrays, the per-block pair lists, masks
+// ~164 B per atom of atom, slot, PME-binning and transfer arrays, the per-block pair lists, masks
 // and work items (~0.5 B per atom per unit of list capacity, the capacity estimated as
 // build_engine does), the PME grids and charge staging (~24 B per grid point), and 8 MiB
 // of fixed overhead.
@@ -498,7 +498,7 @@ size_t engine_bytes_estimate(const fz_system* s) {
   const double a = 1.4 * std::cbrt(32.0 / rho);
   const double vm = a * a * a + 6 * a * a * R + 3 * M_PI * a * R * R + 4.0 / 3.0 * M_PI * R * R * R;
   const double ocap = std::max(256.0, 1.25 * rho * vm);
-  return (size_t)(n * (140.0 + 0.5 * ocap) + 24.0 * K3) + ((size_t)8 << 20);
+  return (size_t)(n * (164.0 + 0.5 * ocap) + 24.0 * K3) + ((size_t)8 << 20);
 }
 
 }  // namespace

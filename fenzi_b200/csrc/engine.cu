@@ -368,7 +368,7 @@ static fz_status build_engine(fz_system* s, int device, void* stream) {
   fz_status r;
   if ((r = e->upload(&e->pos4, pos4)) || (r = e->upload(&e->vel4, vel4)) || (r = e->alloc(&e->pos_build, n)) ||
       (r = e->alloc(&e->facc, 3 * (size_t)n)) || (r = e->alloc(&e->energy, fzk::EN_COUNT)) ||
-      (r = e->alloc(&e->psum, 4)) || (r = e->upload(&e->type, t.type)))
+      (r = e->alloc(&e->psum, 4)) || (r = e->alloc(&e->xfer, 3 * (size_t)n)) || (r = e->upload(&e->type, t.type)))
     return r;
   if (c.consharm) {
     double m0 = 0, m1 = 0;
@@ -1123,10 +1123,12 @@ extern "C" fz_status fz_get_forces(fz_system* s, double* out) {
   if ((r = need_engine(s))) return r;
   if (!out) return fail(FZ_ERR_ARG, "null output");
   Engine* e = s->eng;
-  std::vector<long long> f(3 * (size_t)e->n);
-  if ((r = fz_get_forces_fixed(s, f.data()))) return r;
-  for (int i = 0; i < e->n; ++i)
-    for (int c = 0; c < 3; ++c) out[3 * i + c] = (double)f[(size_t)c * e->n + i] / fzk::kFixFd;
+  // converted on the device and copied straight into the caller's array (230,400 atoms:
+  // 1.40 ms with the conversion on the host; a pinned staging buffer of our own would
+  // cost a new system's first call several ms of allocation)
+  fzk::launch_forces_out(e->facc, e->xfer, e->n, e->st);
+  FZ_CUDA(cudaMemcpyAsync(out, e->xfer, 3 * sizeof(double) * (size_t)e->n, cudaMemcpyDeviceToHost, e->st));
+  FZ_CUDA(cudaStreamSynchronize(e->st));
   return FZ_OK;
 }
 
@@ -1134,17 +1136,18 @@ extern "C" fz_status fz_set_state_f32(fz_system* s, const float* pos, const floa
   fz_status r;
   if ((r = need_engine(s))) return r;
   Engine* e = s->eng;
-  // xyz per atom into the float4 arrays (q and 1/m kept): strided device copies
+  // xyz per atom into the float4 arrays (q and 1/m kept)
+  const size_t bytes = 3 * sizeof(float) * (size_t)e->n;
+  float* x = reinterpret_cast<float*>(e->xfer);
   if (pos) {
-    FZ_CUDA(cudaMemcpy2DAsync(e->pos4, sizeof(float4), pos, 3 * sizeof(float), 3 * sizeof(float), e->n,
-                              cudaMemcpyHostToDevice, e->st));
-    const int one = 1;
-    FZ_CUDA(cudaMemcpyAsync(e->flag, &one, sizeof(int), cudaMemcpyHostToDevice, e->st));
+    FZ_CUDA(cudaMemcpyAsync(x, pos, bytes, cudaMemcpyHostToDevice, e->st));
+    fzk::launch_unpack3(x, e->pos4, e->n, e->flag, e->st);
     e->forces_valid = false;
   }
-  if (vel)
-    FZ_CUDA(cudaMemcpy2DAsync(e->vel4, sizeof(float4), vel, 3 * sizeof(float), 3 * sizeof(float), e->n,
-                              cudaMemcpyHostToDevice, e->st));
+  if (vel) {
+    FZ_CUDA(cudaMemcpyAsync(x + 3 * (size_t)e->n, vel, bytes, cudaMemcpyHostToDevice, e->st));
+    fzk::launch_unpack3(x + 3 * (size_t)e->n, e->vel4, e->n, nullptr, e->st);
+  }
   return FZ_OK;
 }
 
@@ -1152,12 +1155,16 @@ extern "C" fz_status fz_get_state_f32(fz_system* s, float* pos, float* vel) {
   fz_status r;
   if ((r = need_engine(s))) return r;
   Engine* e = s->eng;
-  if (pos)
-    FZ_CUDA(cudaMemcpy2DAsync(pos, 3 * sizeof(float), e->pos4, sizeof(float4), 3 * sizeof(float), e->n,
-                              cudaMemcpyDeviceToHost, e->st));
-  if (vel)
-    FZ_CUDA(cudaMemcpy2DAsync(vel, 3 * sizeof(float), e->vel4, sizeof(float4), 3 * sizeof(float), e->n,
-                              cudaMemcpyDeviceToHost, e->st));
+  const size_t bytes = 3 * sizeof(float) * (size_t)e->n;
+  float* x = reinterpret_cast<float*>(e->xfer);
+  if (pos) {
+    fzk::launch_pack3(e->pos4, x, e->n, e->st);
+    FZ_CUDA(cudaMemcpyAsync(pos, x, bytes, cudaMemcpyDeviceToHost, e->st));
+  }
+  if (vel) {
+    fzk::launch_pack3(e->vel4, x + 3 * (size_t)e->n, e->n, e->st);
+    FZ_CUDA(cudaMemcpyAsync(vel, x + 3 * (size_t)e->n, bytes, cudaMemcpyDeviceToHost, e->st));
+  }
   FZ_CUDA(cudaStreamSynchronize(e->st));
   return FZ_OK;
 }

@@ -127,6 +127,8 @@ struct Engine {
   // PME runs on a second stream concurrently with the pair and bonded kernels
   cudaStream_t st2 = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  // device side of host transfers: 6n floats (positions | velocities) or 3n doubles
+  double* xfer = nullptr;
   // pinned staging
   void* pinned = nullptr;
   size_t pinned_bytes = 0;

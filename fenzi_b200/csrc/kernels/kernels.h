@@ -238,6 +238,12 @@ void launch_reassign(const IntegrateArgs& a, double T, uint64_t seed, uint32_t c
 void launch_restraint(const SysParams& p, const float4* pos4, const int* seg, const float* mass, long long* acc,
                       double inv_m0, double inv_m1, const double* dist, double fc, long long* facc, cudaStream_t st);
 
+// host <-> device state (kernels/state.cu): packed triples to / from float4 arrays, forces
+// in kcal/mol/A to doubles
+void launch_unpack3(const float* in, float4* out, int n, int* flag, cudaStream_t st);
+void launch_pack3(const float4* in, float* out, int n, cudaStream_t st);
+void launch_forces_out(const long long* facc, double* out, int n, cudaStream_t st);
+
 double measure_fp32_peak(int device);
 
 }  // namespace fzk
