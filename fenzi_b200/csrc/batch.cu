@@ -219,8 +219,8 @@ static fz_status build_batch_kernels(fz_batch* b) {
     Engine* e = b->systems[i]->eng;
     rb.push_back(e->rebuild_args());
     nb.push_back(e->nb_args());
-    bd.push_back(e->bonded_args());
-    pme.push_back(e->pme_args());
+    bd.push_back(e->bonded_args(true));
+    pme.push_back(e->pme_args(true));
     if (big_bricks) {
       // a batch has CTAs to spare: bricks as large as the spread's shared region allows
       // (largest divisor of K in [4, 16]) give each spread / gather CTA hundreds of
@@ -320,8 +320,8 @@ static fz_status build_batch_kernels(fz_batch* b) {
   return FZ_OK;
 }
 
-// the batched step: kick/drift (one launch per unit class), outer-list rebuild, then PME
-// on a second stream beside prune, pair and bonded kernels, then kick/RATTLE.  open /
+// the batched step: kick/drift (one launch per unit class), then PME on a second stream
+// beside rebuild, prune, pair and bonded kernels, then kick/RATTLE.  open /
 // close as for the single-system step: inside a chunk graph the kick/RATTLE of a step
 // and the kick/drift of the next are one pass.
 static void batched_step_body(fz_batch* b, cudaStream_t st, bool open = true, bool close = true) {
@@ -330,9 +330,9 @@ static void batched_step_body(fz_batch* b, cudaStream_t st, bool open = true, bo
     if (open) fzk::launch_kick_drift_b(c, st);
     else fzk::launch_close_kick_drift_b(c, st);
   }
-  fzk::launch_rebuild_build_b(k.rb, k.t, st);
   cudaEventRecord(b->ev_fork, st);
   cudaStreamWaitEvent(b->aux, b->ev_fork, 0);
+  fzk::launch_rebuild_build_b(k.rb, k.t, st);
   fzk::launch_pme_b(k.pme, k.t, k.sizes.data(), (int)k.sizes.size(), k.spread_smem, b->aux);
   fzk::launch_rebuild_prune_b(k.rb, k.t, st);
   fzk::launch_nonbonded_b(k.nb, k.t, k.max_ntypes, st);

@@ -218,7 +218,6 @@ static fz_status build_engine(fz_system* s, int device, void* stream) {
     e->own_stream = true;
   }
   FZ_CUDA(cudaStreamCreateWithFlags(&e->st2, cudaStreamNonBlocking));
-  FZ_CUDA(cudaStreamCreateWithFlags(&e->st_cap, cudaStreamNonBlocking));
   {
     // conditional IF nodes for the neighbour kernels inside captured steps: measured
     // ~12 us per step slower on B200 at 230,400 atoms than the flag-checking kernels
@@ -230,6 +229,10 @@ static fz_status build_engine(fz_system* s, int device, void* stream) {
   }
   FZ_CUDA(cudaEventCreateWithFlags(&e->ev_fork, cudaEventDisableTiming));
   FZ_CUDA(cudaEventCreateWithFlags(&e->ev_join, cudaEventDisableTiming));
+  FZ_CUDA(cudaStreamCreateWithFlags(&e->st3, cudaStreamNonBlocking));
+  FZ_CUDA(cudaStreamCreateWithFlags(&e->st_cap, cudaStreamNonBlocking));
+  FZ_CUDA(cudaEventCreateWithFlags(&e->ev_top, cudaEventDisableTiming));
+  FZ_CUDA(cudaEventCreateWithFlags(&e->ev_join3, cudaEventDisableTiming));
   const int n = t.n;
   e->n = n;
   const int nt = (int)t.type_names.size();
@@ -366,10 +369,14 @@ static fz_status build_engine(fz_system* s, int device, void* stream) {
   }
   e->inv_mtot = mt > 0 ? 1.0 / mt : 0.0;
   fz_status r;
-  if ((r = e->upload(&e->pos4, pos4)) || (r = e->upload(&e->vel4, vel4)) || (r = e->alloc(&e->pos_build, n)) ||
-      (r = e->alloc(&e->facc, 3 * (size_t)n)) || (r = e->alloc(&e->energy, fzk::EN_COUNT)) ||
+  if ((r = e->upload(&e->pos4, pos4)) || (r = e->upload(&e->vel4, vel4)) || (r = e->alloc(&e->pos_build, n)) || (r = e->alloc(&e->pos_drift, n)) ||
+      (r = e->alloc(&e->facc, 3 * (size_t)n)) || (r = e->alloc(&e->energy, sizeof(Engine::Readback) / sizeof(long long))) ||
       (r = e->alloc(&e->psum, 4)) || (r = e->alloc(&e->xfer, 3 * (size_t)n)) || (r = e->upload(&e->type, t.type)))
     return r;
+  static_assert(sizeof(Engine::Readback) == sizeof(long long) * fzk::EN_COUNT + sizeof(int) * (fzk::CNT_COUNT + 2),
+                "the readback block is packed");
+  e->counters = reinterpret_cast<int*>(e->energy + fzk::EN_COUNT);
+  e->status = e->counters + fzk::CNT_COUNT;
   if (c.consharm) {
     double m0 = 0, m1 = 0;
     for (int i = 0; i < n; ++i) {
@@ -398,7 +405,7 @@ static fz_status build_engine(fz_system* s, int device, void* stream) {
       (r = e->alloc(&e->inner_m, (size_t)ngrp * (e->ocap / 32))) || (r = e->alloc(&e->dmask, (size_t)nblk * 32)) ||
       (r = e->alloc(&e->masks, (size_t)e->mask_cap * fzk::kIG)) || (r = e->alloc(&e->pos_prune, n)) ||
       (r = e->alloc(&e->flag_prune, 1)) || (r = e->alloc(&e->items, (size_t)ngrp * (e->ocap / 32 + 1))) ||
-      (r = e->alloc(&e->flag, 1)) || (r = e->alloc(&e->counters, fzk::CNT_COUNT)) || (r = e->alloc(&e->status, 1)))
+      (r = e->alloc(&e->flag, 1)))
     return r;
   {
     // the permanent dummy slot (last) used to pad partial tiles: far away, q = 0, padding type
@@ -427,48 +434,8 @@ static fz_status build_engine(fz_system* s, int device, void* stream) {
     if ((size_t)nt1 * nt1 * sizeof(float2) > 200 * 1024) return fail(FZ_ERR_ARG, "too many LJ types");
     if ((r = e->upload(&e->ljtab, lj)) || (r = e->upload(&e->lj14, l14))) return r;
   }
-  // ---- bonded arrays
-  {
-    std::vector<int2> b, u, x, q14;
-    std::vector<int4> an, dh, im;
-    std::vector<float2> bp, ap, up, ip;
-    std::vector<float4> dp;
-    for (size_t k = 0; k < t.bond_k.size(); ++k) {
-      b.push_back(make_int2(t.bond[2 * k], t.bond[2 * k + 1]));
-      bp.push_back(make_float2((float)t.bond_k[k], (float)t.bond_r0[k]));
-    }
-    for (size_t k = 0; k < t.angle_k.size(); ++k) {
-      an.push_back(make_int4(t.angle[3 * k], t.angle[3 * k + 1], t.angle[3 * k + 2], 0));
-      ap.push_back(make_float2((float)t.angle_k[k], (float)t.angle_t0[k]));
-    }
-    for (size_t k = 0; k < t.ub_k.size(); ++k) {
-      u.push_back(make_int2(t.ub[2 * k], t.ub[2 * k + 1]));
-      up.push_back(make_float2((float)t.ub_k[k], (float)t.ub_r0[k]));
-    }
-    for (size_t k = 0; k < t.dihe_k.size(); ++k) {
-      dh.push_back(make_int4(t.dihe[4 * k], t.dihe[4 * k + 1], t.dihe[4 * k + 2], t.dihe[4 * k + 3]));
-      dp.push_back(make_float4((float)t.dihe_k[k], (float)t.dihe_n[k], (float)std::cos(t.dihe_d[k]),
-                               (float)std::sin(t.dihe_d[k])));
-    }
-    for (size_t k = 0; k < t.impr_k.size(); ++k) {
-      im.push_back(make_int4(t.impr[4 * k], t.impr[4 * k + 1], t.impr[4 * k + 2], t.impr[4 * k + 3]));
-      ip.push_back(make_float2((float)t.impr_k[k], (float)t.impr_p0[k]));
-    }
-    for (size_t k = 0; k < t.excl_pairs.size() / 2; ++k) x.push_back(make_int2(t.excl_pairs[2 * k], t.excl_pairs[2 * k + 1]));
-    for (size_t k = 0; k < t.p14_pairs.size() / 2; ++k) q14.push_back(make_int2(t.p14_pairs[2 * k], t.p14_pairs[2 * k + 1]));
-    e->nbond = (int)b.size();
-    e->nangle = (int)an.size();
-    e->nub = (int)u.size();
-    e->ndihe = (int)dh.size();
-    e->nimpr = (int)im.size();
-    e->nexcl = (int)x.size();
-    e->n14 = (int)q14.size();
-    if ((r = e->upload(&e->bond, b)) || (r = e->upload(&e->bond_prm, bp)) || (r = e->upload(&e->angle, an)) ||
-        (r = e->upload(&e->angle_prm, ap)) || (r = e->upload(&e->ub, u)) || (r = e->upload(&e->ub_prm, up)) ||
-        (r = e->upload(&e->dihe, dh)) || (r = e->upload(&e->dihe_prm, dp)) || (r = e->upload(&e->impr, im)) ||
-        (r = e->upload(&e->impr_prm, ip)) || (r = e->upload(&e->excl, x)) || (r = e->upload(&e->p14, q14)))
-      return r;
-  }
+  std::vector<int4> unit_atoms;
+  int n33 = 0;  // units of three atoms and three constraints
   // ---- integration units: free atoms first, then clusters (by size)
   {
     // clusters whose atoms are all fixed need no constraint solve: free units
@@ -479,7 +446,7 @@ static fz_status build_engine(fz_system* s, int device, void* stream) {
       if (!all_fixed)
         for (int k = 0; k < cl.na; ++k) in_cl[cl.atom[k]] = 1;
     }
-    std::vector<int4> ua;
+    std::vector<int4>& ua = unit_atoms;
     std::vector<int> um;
     std::vector<float4> ud;
     // grouped by class (atoms, constraints): each class is one integrator launch with
@@ -528,14 +495,14 @@ static fz_status build_engine(fz_system* s, int device, void* stream) {
       return false;
     };
     {
-      int n33 = 0, ntri = 0;
+      int n33c = 0, ntri = 0;
       Cluster tmp;
       for (const auto& cl : t.clusters)
         if (cl.na == 3 && cl.nc == 3 && in_cl[cl.atom[0]]) {
-          ++n33;
+          ++n33c;
           ntri += as_triangle(cl, tmp) ? 1 : 0;
         }
-      e->settle = (n33 > 0 && ntri == n33) ? 1 : 0;
+      e->settle = (n33c > 0 && ntri == n33c) ? 1 : 0;
       if (const char* v = std::getenv("FZ_SETTLE")) e->settle = e->settle && std::atoi(v) != 0;
     }
     for (int na = 2; na <= 4; ++na)
@@ -553,7 +520,119 @@ static fz_status build_engine(fz_system* s, int device, void* stream) {
         }
     e->nunits = (int)ua.size();
     e->cls_begin[e->ncls] = e->nunits;
+    for (int k = 0; k < e->ncls; ++k)
+      if (e->cls_na[k] == 3 && e->cls_nc[k] == 3) {
+        e->unit_term_begin = e->cls_begin[k];
+        n33 = e->cls_begin[k + 1] - e->cls_begin[k];
+      }
     if ((r = e->upload(&e->unit_atoms, ua)) || (r = e->upload(&e->unit_meta, um)) || (r = e->upload(&e->unit_d, ud)))
+      return r;
+  }
+  // ---- bonded arrays: of the bonds, angles and exclusion pairs, those inside a SETTLE
+  // water that fit its term set come last (the integrator evaluates them in a step)
+  {
+    std::vector<int2> b, u, x, q14;
+    std::vector<int4> an, dh, im;
+    std::vector<float2> bp, ap, up, ip;
+    std::vector<float4> dp;
+    const int wbase = e->unit_term_begin, nwat = e->settle ? n33 : 0;
+    std::vector<int> wat(n, -1), loc(n, 0);
+    for (int u = 0; u < nwat; ++u) {
+      const int a[3] = {unit_atoms[wbase + u].x, unit_atoms[wbase + u].y, unit_atoms[wbase + u].z};
+      for (int k = 0; k < 3; ++k) {
+        wat[a[k]] = u;
+        loc[a[k]] = k;
+      }
+    }
+    std::vector<fzk::UnitTerms> ut(nwat);
+    if (nwat) std::memset(ut.data(), 0, sizeof(fzk::UnitTerms) * nwat);
+    // takes bit `bit` of the unit of atoms i and j (one term of each slot), -1 if not inside one
+    auto take = [&](int i, int j, int bit) {
+      if (wat[i] < 0 || wat[i] != wat[j] || i == j || (ut[wat[i]].has >> bit & 1)) return -1;
+      ut[wat[i]].has |= 1 << bit;
+      return wat[i];
+    };
+    auto slot = [&](int i, int j) { return loc[i] + loc[j] - 1; };  // (0,1) 0, (0,2) 1, (1,2) 2
+    std::vector<char> bin(t.bond_k.size(), 0), ain(t.angle_k.size(), 0), xin(t.excl_pairs.size() / 2, 0);
+    for (size_t k = 0; k < bin.size(); ++k) {
+      const int i = t.bond[2 * k], j = t.bond[2 * k + 1], u = take(i, j, slot(i, j));
+      if (u < 0) continue;
+      bin[k] = 1;
+      ut[u].bond[slot(i, j)] = make_float2((float)t.bond_k[k], (float)t.bond_r0[k]);
+    }
+    for (size_t k = 0; k < ain.size(); ++k) {
+      const int i = t.angle[3 * k], c0 = t.angle[3 * k + 1], j = t.angle[3 * k + 2];
+      if (loc[c0] != 0 || wat[c0] < 0 || wat[c0] != wat[i] || i == c0 || j == c0) continue;
+      const int u = take(i, j, 3);
+      if (u < 0) continue;
+      ain[k] = 1;
+      if (loc[i] == 2) ut[u].has |= 16;
+      ut[u].angle = make_float2((float)t.angle_k[k], (float)t.angle_t0[k]);
+    }
+    for (size_t k = 0; k < xin.size(); ++k) {
+      const int i = t.excl_pairs[2 * k], j = t.excl_pairs[2 * k + 1];
+      if (take(i, j, 5 + slot(i, j)) >= 0) xin[k] = 1;
+    }
+    if (nwat) {
+      // few different term sets: a table and an index per water
+      std::map<std::string, int> seen;
+      std::vector<fzk::UnitTerms> table;
+      std::vector<int> of(nwat);
+      for (int u = 0; u < nwat; ++u) {
+        const std::string key((const char*)&ut[u], sizeof(ut[u]));
+        auto it = seen.find(key);
+        if (it == seen.end()) {
+          it = seen.emplace(key, (int)table.size()).first;
+          table.push_back(ut[u]);
+        }
+        of[u] = it->second;
+      }
+      if ((r = e->upload(&e->unit_terms, table)) || (r = e->upload(&e->unit_term_of, of))) return r;
+    }
+    for (int last = 0; last < 2; ++last) {
+    for (size_t k = 0; k < t.bond_k.size(); ++k) {
+      if (bin[k] != last) continue;
+      b.push_back(make_int2(t.bond[2 * k], t.bond[2 * k + 1]));
+      bp.push_back(make_float2((float)t.bond_k[k], (float)t.bond_r0[k]));
+    }
+    for (size_t k = 0; k < t.angle_k.size(); ++k) {
+      if (ain[k] != last) continue;
+      an.push_back(make_int4(t.angle[3 * k], t.angle[3 * k + 1], t.angle[3 * k + 2], 0));
+      ap.push_back(make_float2((float)t.angle_k[k], (float)t.angle_t0[k]));
+    }
+    for (size_t k = 0; k < t.excl_pairs.size() / 2; ++k)
+      if (xin[k] == last) x.push_back(make_int2(t.excl_pairs[2 * k], t.excl_pairs[2 * k + 1]));
+    if (!last) {
+      e->nbond_step = (int)b.size();
+      e->nangle_step = (int)an.size();
+      e->nexcl_step = (int)x.size();
+    }
+    }
+    for (size_t k = 0; k < t.ub_k.size(); ++k) {
+      u.push_back(make_int2(t.ub[2 * k], t.ub[2 * k + 1]));
+      up.push_back(make_float2((float)t.ub_k[k], (float)t.ub_r0[k]));
+    }
+    for (size_t k = 0; k < t.dihe_k.size(); ++k) {
+      dh.push_back(make_int4(t.dihe[4 * k], t.dihe[4 * k + 1], t.dihe[4 * k + 2], t.dihe[4 * k + 3]));
+      dp.push_back(make_float4((float)t.dihe_k[k], (float)t.dihe_n[k], (float)std::cos(t.dihe_d[k]),
+                               (float)std::sin(t.dihe_d[k])));
+    }
+    for (size_t k = 0; k < t.impr_k.size(); ++k) {
+      im.push_back(make_int4(t.impr[4 * k], t.impr[4 * k + 1], t.impr[4 * k + 2], t.impr[4 * k + 3]));
+      ip.push_back(make_float2((float)t.impr_k[k], (float)t.impr_p0[k]));
+    }
+    for (size_t k = 0; k < t.p14_pairs.size() / 2; ++k) q14.push_back(make_int2(t.p14_pairs[2 * k], t.p14_pairs[2 * k + 1]));
+    e->nbond = (int)b.size();
+    e->nangle = (int)an.size();
+    e->nub = (int)u.size();
+    e->ndihe = (int)dh.size();
+    e->nimpr = (int)im.size();
+    e->nexcl = (int)x.size();
+    e->n14 = (int)q14.size();
+    if ((r = e->upload(&e->bond, b)) || (r = e->upload(&e->bond_prm, bp)) || (r = e->upload(&e->angle, an)) ||
+        (r = e->upload(&e->angle_prm, ap)) || (r = e->upload(&e->ub, u)) || (r = e->upload(&e->ub_prm, up)) ||
+        (r = e->upload(&e->dihe, dh)) || (r = e->upload(&e->dihe_prm, dp)) || (r = e->upload(&e->impr, im)) ||
+        (r = e->upload(&e->impr_prm, ip)) || (r = e->upload(&e->excl, x)) || (r = e->upload(&e->p14, q14)))
       return r;
   }
   // ---- PME
@@ -572,14 +651,16 @@ static fz_status build_engine(fz_system* s, int device, void* stream) {
       const int Kd = e->K[d];
       std::vector<float2> tw(Kd);
       std::vector<float> g(Kd), ff(Kd);
+      std::vector<double> bm(Kd);
       for (int m = 0; m < Kd; ++m) {
         const double ang = -2.0 * M_PI * m / Kd;
         tw[m] = make_float2((float)std::cos(ang), (float)std::sin(ang));
         const double f = (m <= Kd / 2 ? m : m - Kd) / c.box[d];
         ff[m] = (float)(f * f);
-        g[m] = (float)(bmod2(m, Kd) * std::exp(-M_PI * M_PI * f * f / b2));
+        bm[m] = bmod2(m, Kd);
+        g[m] = (float)(bm[m] * std::exp(-M_PI * M_PI * f * f / b2));
       }
-      if ((r = e->upload(&e->tw[d], tw)) || (r = e->upload(&e->gfac[d], g)) || (r = e->upload(&e->f2[d], ff))) return r;
+      if ((r = e->upload(&e->bm2[d], bm)) || (r = e->upload(&e->tw[d], tw)) || (r = e->upload(&e->gfac[d], g)) || (r = e->upload(&e->f2[d], ff))) return r;
     }
     e->gscale = (float)(kCC / (M_PI * V));
   }
@@ -682,32 +763,29 @@ fz_status set_box(Engine* e, double L) {
   e->dcy = std::min(e->ncy, (int)std::ceil(e->plist / (e->box_d[1] / e->ncy)));
   const double colw = std::max(e->box_d[0] / e->ncx, e->box_d[1] / e->ncy);
   e->all_images = (0.5 * lmin < e->plist + 3.0 * std::max(colw, e->col_a)) ? 1 : 0;
-  const int ktot = e->K[0] + e->K[1] + e->K[2];
-  if (!e->pme_tab_host) FZ_CUDA(cudaMallocHost(&e->pme_tab_host, sizeof(float) * 2 * ktot));
-  // the previous step's table copies have completed: barostat steps synchronise each step
-  const double b2 = (double)p.beta * (double)p.beta;
-  float* h = e->pme_tab_host;
+  // the influence tables of the new box, made on the device (queued after the last
+  // step's PME; as host tables they were six copies a step)
+  fzk::PmeTables t{};
   for (int d = 0; d < 3; ++d) {
-    const int Kd = e->K[d];
-    float* g = h;
-    float* ff = h + Kd;
-    for (int m = 0; m < Kd; ++m) {
-      const double f = (m <= Kd / 2 ? m : m - Kd) / e->box_d[d];
-      ff[m] = (float)(f * f);
-      g[m] = (float)(bmod2(m, Kd) * std::exp(-M_PI * M_PI * f * f / b2));
-    }
-    FZ_CUDA(cudaMemcpyAsync(e->gfac[d], g, sizeof(float) * Kd, cudaMemcpyHostToDevice, e->st));
-    FZ_CUDA(cudaMemcpyAsync(e->f2[d], ff, sizeof(float) * Kd, cudaMemcpyHostToDevice, e->st));
-    h += 2 * Kd;
+    t.K[d] = e->K[d];
+    t.bm2[d] = e->bm2[d];
+    t.gfac[d] = e->gfac[d];
+    t.f2[d] = e->f2[d];
+    t.box[d] = e->box_d[d];
   }
+  t.beta = (double)p.beta;
+  fzk::launch_pme_tables(t, e->st);
+  FZ_CUDA(cudaGetLastError());
   return FZ_OK;
 }
 
 // host copy of the energy slots and the cumulative list counters (synchronises)
 static fz_status read_slots(Engine* e, long long* en, int* cnt) {
-  FZ_CUDA(cudaMemcpyAsync(en, e->energy, sizeof(long long) * fzk::EN_COUNT, cudaMemcpyDeviceToHost, e->st));
-  if (cnt) FZ_CUDA(cudaMemcpyAsync(cnt, e->counters, sizeof(int) * fzk::CNT_COUNT, cudaMemcpyDeviceToHost, e->st));
-  return e->check();
+  Engine::Readback b;
+  const fz_status r = e->read_back(&b);
+  std::memcpy(en, b.energy, sizeof(b.energy));
+  if (cnt) std::memcpy(cnt, b.counters, sizeof(b.counters));
+  return r;
 }
 
 static double volume(const Engine* e) { return e->box_d[0] * e->box_d[1] * e->box_d[2]; }
@@ -767,6 +845,7 @@ static fz_status npt_step(Engine* e) {
     FZ_CUDA(cudaMemcpyAsync(e->flag_prune, &one, sizeof(int), cudaMemcpyHostToDevice, e->st));
   FZ_CUDA(cudaMemsetAsync(e->energy, 0, fzk::EN_COUNT * sizeof(long long), e->st));
   fzk::IntegrateArgs ia = e->int_args();
+  ia.fuse_terms = 0;  // the evaluation below takes all terms (energies and virial)
   ia.lam = Ln / L;
   ia.vfric = std::exp(-0.5 * dt * e->Ldot / L);
   fzk::launch_kick_drift_npt(ia, e->st);
@@ -871,11 +950,11 @@ extern "C" fz_status fz_step(fz_system* s, int nsteps) {
     } else {
       e->mark(0);
       fzk::launch_kick_drift(ia, e->st);
-      e->forces(false);
+      e->forces(false, FZ_TERM_ALL, true);
       fzk::launch_kick_rattle(ia, false, true, e->st);
       e->mark(6);
       if (e->timing) e->collect_step();
-      e->launches += 2 * e->ncls;
+      e->launches += fzk::drift_launches(ia) + e->ncls;
     }
     e->step++;
     if (e->temp_reset_every > 0 && e->step % e->temp_reset_every == 0) {

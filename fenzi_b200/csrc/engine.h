@@ -61,6 +61,14 @@ struct Engine {
   // consharm restraint: segment of every atom (0, 1, -1), masses, fixed-point mass
   // centre sums (x0 y0 z0 x1 y1 z1), inverse segment masses, target offset, constant
   bool restraint = false;
+  // of each kind of bonded term, the first *_step are those the bonded kernel evaluates in
+  // a step (the rest belong to rigid waters: the integrator's pass has them, see
+  // UnitTerms); a force evaluation outside a step takes all
+  int nbond_step = 0, nangle_step = 0, nexcl_step = 0;
+  fzk::UnitTerms* unit_terms = nullptr;
+  int* unit_term_of = nullptr;
+  int unit_term_begin = 0;
+  float4* pos_drift = nullptr;  // drifted positions of this step, never wrapped by a rebuild
   int* rs_seg = nullptr;
   float* rs_mass = nullptr;
   long long* rs_acc = nullptr;
@@ -127,6 +135,9 @@ struct Engine {
   // PME runs on a second stream concurrently with the pair and bonded kernels
   cudaStream_t st2 = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  // bonded terms outside rigid waters on a third
+  cudaStream_t st3 = nullptr;
+  cudaEvent_t ev_top = nullptr, ev_join3 = nullptr;
   // device side of host transfers: 6n floats (positions | velocities) or 3n doubles
   double* xfer = nullptr;
   // pinned staging
@@ -145,7 +156,7 @@ struct Engine {
   double plist = 0.0, cutoff = 0.0, col_a = 0.0;
   float skin_half2_nve = 0.f, prune_half2_nve = 0.f;
   double prune_delta = 0.0;
-  float* pme_tab_host = nullptr;  // pinned: gfac|f2 per dimension
+  double* bm2[3] = {nullptr, nullptr, nullptr};  // per dimension: |b(m)|^2 of the splines
   int ncx = 1, ncy = 1;
 
   template <class T>
@@ -193,13 +204,15 @@ struct Engine {
     if (chunk_graph) cudaGraphDestroy(chunk_graph);
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
-    if (st2) cudaStreamDestroy(st2);
+    if (ev_top) cudaEventDestroy(ev_top);
+    if (ev_join3) cudaEventDestroy(ev_join3);
+    if (st3) cudaStreamDestroy(st3);
     if (st_cap) cudaStreamDestroy(st_cap);
+    if (st2) cudaStreamDestroy(st2);
     for (auto& x : ev)
       if (x) cudaEventDestroy(x);
     for (void* p : allocs) cudaFree(p);
     if (pinned) cudaFreeHost(pinned);
-    if (pme_tab_host) cudaFreeHost(pme_tab_host);
     if (own_stream && st) cudaStreamDestroy(st);
   }
 
@@ -276,10 +289,11 @@ struct Engine {
     a.minb = nb_per_sm;
     return a;
   }
-  fzk::PmeArgs pme_args() const {
+  // step: the forces of a step, after its drift (pos_drift)
+  fzk::PmeArgs pme_args(bool step = false) const {
     fzk::PmeArgs a{};
     a.p = p;
-    a.pos4 = pos4;
+    a.pos4 = step ? pos_drift : pos4;
     a.n = n;
     for (int d = 0; d < 3; ++d) {
       a.K[d] = K[d];
@@ -303,16 +317,16 @@ struct Engine {
     a.gather = gather_mode;
     return a;
   }
-  fzk::BondedArgs bonded_args() const {
+  fzk::BondedArgs bonded_args(bool step = false) const {
     fzk::BondedArgs a{};
     a.p = p;
-    a.pos4 = pos4;
-    a.nbond = nbond;
-    a.nangle = nangle;
+    a.pos4 = step ? pos_drift : pos4;
+    a.nbond = step ? nbond_step : nbond;
+    a.nangle = step ? nangle_step : nangle;
     a.nub = nub;
     a.ndihe = ndihe;
     a.nimpr = nimpr;
-    a.nexcl = nexcl;
+    a.nexcl = step ? nexcl_step : nexcl;
     a.n14 = n14;
     a.bond = bond;
     a.bond_prm = bond_prm;
@@ -340,6 +354,11 @@ struct Engine {
     a.unit_meta = unit_meta;
     a.unit_d = unit_d;
     a.pos4 = pos4;
+    a.pos_drift = pos_drift;
+    a.unit_terms = unit_terms;
+    a.unit_term_of = unit_term_of;
+    a.unit_term_begin = unit_term_begin;
+    a.fuse_terms = unit_terms ? 1 : 0;
     a.vel4 = vel4;
     a.facc = facc;
     a.xyzq_s = xyzq_s;
@@ -376,18 +395,27 @@ struct Engine {
   void mark(int k) {
     if (timing) cudaEventRecord(ev[k], st);
   }
-  void forces(bool energies, int terms = FZ_TERM_ALL) {
+  // step: after a drift whose pass has evaluated the rigid waters' own terms
+  void forces(bool energies, int terms = FZ_TERM_ALL, bool step = false) {
     mark(1);
     fzk::launch_rebuild(rebuild_args(), st);
     launches += fzk::kRebuildBuildLaunches + fzk::kRebuildPruneLaunches;
     mark(2);
+    // PME beside the pair and bonded kernels (in line when the stages are timed)
+    const bool beside = (terms & FZ_TERM_PME) && st2 && !timing;
+    if (beside) {
+      cudaEventRecord(ev_fork, st);
+      cudaStreamWaitEvent(st2, ev_fork, 0);
+      fzk::launch_pme(pme_args(step), energies, st2);
+      cudaEventRecord(ev_join, st2);
+    }
     if (terms & FZ_TERM_NONBONDED) {
       fzk::launch_nonbonded(nb_args(), energies, st);
       launches += 1;
     }
     mark(3);
     if (terms & (FZ_TERM_BONDED | FZ_TERM_BONDED_PARTS)) {
-      fzk::BondedArgs a = bonded_args();
+      fzk::BondedArgs a = bonded_args(step);
       if (!(terms & FZ_TERM_BONDED)) {
         // selected parts only: the kernel's flattened term range skips empty classes
         if (!(terms & FZ_TERM_BONDS)) a.nbond = 0;
@@ -399,7 +427,7 @@ struct Engine {
         if (!(terms & FZ_TERM_EXCLUSIONS)) a.nexcl = 0;
       }
       fzk::launch_bonded(a, energies, st);
-      launches += bonded_launches();
+      launches += step ? bonded_step_launches() : bonded_launches();
     }
     if ((terms & FZ_TERM_BONDED) && restraint) {
       restraint_forces(st);
@@ -407,7 +435,8 @@ struct Engine {
     }
     mark(4);
     if (terms & FZ_TERM_PME) {
-      fzk::launch_pme(pme_args(), energies, st);
+      if (beside) cudaStreamWaitEvent(st, ev_join, 0);
+      else fzk::launch_pme(pme_args(step), energies, st);
       launches += fzk::pme_launches(pme_args());
     }
     mark(5);
@@ -494,10 +523,14 @@ struct Engine {
     rebuild_build_step();
     prune_step();
   }
-  // kernels one captured step launches besides the conditional bodies
+  // kernels one captured step launches
   long long graph_step_launches() const {
-    return 2 * ncls + (cond_graph ? 2 : fzk::kRebuildBuildLaunches + fzk::kRebuildPruneLaunches) + 1 +
-           bonded_launches() + fzk::pme_launches(pme_args()) + (restraint ? 2 : 0);
+    return fzk::drift_launches(int_args()) + ncls +
+           (cond_graph ? 2 : fzk::kRebuildBuildLaunches + fzk::kRebuildPruneLaunches) + 1 + bonded_step_launches() +
+           fzk::pme_launches(pme_args()) + (restraint ? 2 : 0);
+  }
+  int bonded_step_launches() const {
+    return (nbond_step + nangle_step + nub + ndihe + nimpr + nexcl_step + n14 > 0) ? 1 : 0;
   }
   int bonded_launches() const { return (nbond + nangle + nub + ndihe + nimpr + nexcl + n14 > 0) ? 1 : 0; }
   // launches of the conditional bodies (per rebuild and per prune) since the last
@@ -510,61 +543,45 @@ struct Engine {
     seen_rb_launch = cnt[fzk::CNT_REBUILDS];
     seen_pr_launch = cnt[fzk::CNT_PRUNES];
   }
-  // forces with PME on st2, overlapping the pair and bonded kernels on st
-  // (PME needs only the positions, so it starts before the prune and overlaps it too)
-  void forces_overlapped() {
-    rebuild_build_step();
-    cudaEventRecord(ev_fork, st);
-    cudaStreamWaitEvent(st2, ev_fork, 0);
-    fzk::launch_pme(pme_args(), false, st2);
-    prune_step();
-    fzk::launch_nonbonded(nb_args(), false, st);
-    fzk::launch_bonded(bonded_args(), false, st);
-    if (restraint) restraint_forces(st);
-    cudaEventRecord(ev_join, st2);
-    cudaStreamWaitEvent(st, ev_join, 0);
-  }
-  // One integrator pass over all unit classes; with a second stream the first class
-  // (free atoms) runs beside the others: classes touch disjoint atoms.
-  template <class L>
-  void integrate_classes(const fzk::IntegrateArgs& ia, L launch) {
-    if (!st2 || ia.ncls < 2) {
-      launch(ia, st);
-      return;
-    }
-    fzk::IntegrateArgs first = ia, rest = ia;
-    first.ncls = 1;
-    rest.ncls = ia.ncls - 1;
-    for (int c = 0; c < rest.ncls; ++c) {
-      rest.cls_na[c] = ia.cls_na[c + 1];
-      rest.cls_nc[c] = ia.cls_nc[c + 1];
-      rest.cls_begin[c] = ia.cls_begin[c + 1];
-    }
-    rest.cls_begin[rest.ncls] = ia.cls_begin[ia.ncls];
-    cudaEventRecord(ev_fork, st);
-    cudaStreamWaitEvent(st2, ev_fork, 0);
-    launch(first, st2);
-    launch(rest, st);
-    cudaEventRecord(ev_join, st2);
-    cudaStreamWaitEvent(st, ev_join, 0);
-  }
   // One MD step.  open: the step starts with its own kick + drift pass (else the
   // previous step left its closing kick + RATTLE to this step's first pass); close: the
   // step ends with the kick + RATTLE pass (else the next step's first pass does it).
+  //
+  // PME runs on st2 beside the pair kernel, the bonded terms outside rigid waters on
+  // st3.  Both read pos_drift, which a rebuild does not wrap, so they need only the
+  // drift and start beside the neighbour launches: the step's length is the longer of
+  // the two chains.
   void step_body(bool open = true, bool close = true) {
     const fzk::IntegrateArgs ia = int_args();
-    if (open)
-      integrate_classes(ia, [](const fzk::IntegrateArgs& a, cudaStream_t s) { fzk::launch_kick_drift(a, s); });
-    else
-      integrate_classes(ia, [](const fzk::IntegrateArgs& a, cudaStream_t s) { fzk::launch_close_kick_drift(a, s); });
-    if (st2)
-      forces_overlapped();
-    else
-      forces(false);
-    if (close)
-      integrate_classes(ia, [](const fzk::IntegrateArgs& a, cudaStream_t s) {
-        fzk::launch_kick_rattle(a, false, true, s);
-      });
+    if (!st2) {
+      if (open) fzk::launch_kick_drift(ia, st);
+      else fzk::launch_close_kick_drift(ia, st);
+      forces(false, FZ_TERM_ALL, true);
+      if (close) fzk::launch_kick_rattle(ia, false, true, st);
+      return;
+    }
+    const fzk::PmeArgs pa = pme_args(true);
+    cudaEventRecord(ev_top, st);
+    cudaStreamWaitEvent(st2, ev_top, 0);
+    fzk::launch_pme_clear(pa, st2);
+    if (open) fzk::launch_kick_drift(ia, st);
+    else fzk::launch_close_kick_drift(ia, st);
+    cudaEventRecord(ev_fork, st);
+    cudaStreamWaitEvent(st2, ev_fork, 0);
+    fzk::launch_pme(pa, false, st2, true);
+    const bool bonded = bonded_step_launches() > 0;
+    if (bonded) {
+      cudaStreamWaitEvent(st3, ev_fork, 0);
+      fzk::launch_bonded(bonded_args(true), false, st3);
+      cudaEventRecord(ev_join3, st3);
+    }
+    rebuild_step();
+    fzk::launch_nonbonded(nb_args(), false, st);
+    if (restraint) restraint_forces(st);
+    if (bonded) cudaStreamWaitEvent(st, ev_join3, 0);
+    cudaEventRecord(ev_join, st2);
+    cudaStreamWaitEvent(st, ev_join, 0);
+    if (close) fzk::launch_kick_rattle(ia, false, true, st);
   }
   fz_status graph_step() {
     if (!step_exec) {
@@ -616,14 +633,25 @@ struct Engine {
     chunk_exec = nullptr;
     chunk_graph = nullptr;
   }
-  fz_status check() {
-    int h = 0;
-    int cnt[fzk::CNT_COUNT];
-    FZ_CUDA(cudaMemcpyAsync(&h, status, sizeof(int), cudaMemcpyDeviceToHost, st));
-    FZ_CUDA(cudaMemcpyAsync(cnt, counters, sizeof(cnt), cudaMemcpyDeviceToHost, st));
+  // what the host reads back after a call: energy slots, list counters and the status
+  // word lie together on the device, one copy (and one wait) brings them
+  struct Readback {
+    long long energy[fzk::EN_COUNT];
+    int counters[fzk::CNT_COUNT];
+    int status, pad;
+  };
+  fz_status read_back(Readback* b) {
+    FZ_CUDA(cudaMemcpyAsync(b, energy, sizeof(Readback), cudaMemcpyDeviceToHost, st));
     FZ_CUDA(cudaStreamSynchronize(st));
     FZ_CUDA(cudaGetLastError());
-    account_conditional(cnt);
+    account_conditional(b->counters);
+    return status_of(b->status);
+  }
+  fz_status check() {
+    Readback b;
+    return read_back(&b);
+  }
+  static fz_status status_of(int h) {
     if (h) {
       std::string m = "device status:";
       if (h & fzk::ST_TILE_OVERFLOW) m += " pair-tile capacity exceeded;";

@@ -10,24 +10,12 @@
 // evaluated in FP64 (it cancels against the self term and the reciprocal sum).
 // Dihedrals use the exact CHARMM form K(1 + cos(n phi - delta)) for any delta (the
 // reference's sin(n phi - delta) update at :364-365 is right only for delta in {0, 180}).
+#include "bonded_terms.cuh"
 #include "common.cuh"
 #include "kernels.h"
 
 namespace fzk {
 
-// minimum-image difference a - b of two FP32 positions, formed in FP64 and rounded once:
-// two atoms of a term split by the periodic boundary are about L apart before the image
-// shift, and an FP32 difference would round at the ulp of L (up to 3.8e-6 A for
-// L = 130 A), a 1e-4 relative error in the force of a stiff bond
-__device__ __forceinline__ float3 image_diff(float4 a, float4 b, const SysParams& p) {
-  double d[3] = {(double)a.x - (double)b.x, (double)a.y - (double)b.y, (double)a.z - (double)b.z};
-  min_image_d(d, p);
-  return make_float3((float)d[0], (float)d[1], (float)d[2]);
-}
-__device__ __forceinline__ float dot(float3 a, float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-__device__ __forceinline__ float3 cross(float3 a, float3 b) {
-  return make_float3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
-}
 __device__ __forceinline__ void addf(long long* facc, int n, int i, float3 f) {
   red_add(facc + i, to_fix(f.x));
   red_add(facc + n + i, to_fix(f.y));
@@ -76,9 +64,8 @@ __device__ __forceinline__ void bonded_body(const BondedArgs& a, int bid) {
     const int2 b = a.bond[r];
     const float2 pr = a.bond_prm[r];
     const float3 d = image_diff(a.pos4[b.x], a.pos4[b.y], p);
-    const float rr = sqrtf(dot(d, d));
-    const float dr = rr - pr.y;
-    const float f = rr > 0.f ? -2.f * pr.x * dr / rr : 0.f;
+    float dr;
+    const float f = bond_force(d, pr, &dr);
     addf(a.facc, n, b.x, make_float3(f * d.x, f * d.y, f * d.z));
     addf(a.facc, n, b.y, make_float3(-f * d.x, -f * d.y, -f * d.z));
     if (ENERGY) {
@@ -93,21 +80,9 @@ __device__ __forceinline__ void bonded_body(const BondedArgs& a, int bid) {
     const float4 rj = a.pos4[q.y];
     const float3 u = image_diff(a.pos4[q.x], rj, p);
     const float3 v = image_diff(a.pos4[q.z], rj, p);
-    const float uu = dot(u, u), vv = dot(v, v), uv = dot(u, v);
-    const float3 uxv = cross(u, v);
-    const float ruv = rsqrtf(uu * vv);
-    const float c = uv * ruv;
-    const float s = sqrtf(dot(uxv, uxv)) * ruv;
-    const float th = atan2f(s, c);
-    const float dth = th - pr.y;
-    const float dE = 2.f * pr.x * dth;
-    const float sf = fmaxf(s, 1e-6f);
-    const float k1 = -dE / sf;
-    // dtheta/du = -(v/(|u||v|) - c u/|u|^2)/sin ; force = -dE * dtheta/du
-    const float3 gu = make_float3(v.x * ruv - c * u.x / uu, v.y * ruv - c * u.y / uu, v.z * ruv - c * u.z / uu);
-    const float3 gv = make_float3(u.x * ruv - c * v.x / vv, u.y * ruv - c * v.y / vv, u.z * ruv - c * v.z / vv);
-    const float3 fi = make_float3(-k1 * gu.x, -k1 * gu.y, -k1 * gu.z);
-    const float3 fk = make_float3(-k1 * gv.x, -k1 * gv.y, -k1 * gv.z);
+    float3 fi, fk;
+    float dth;
+    angle_force(u, v, pr, &fi, &fk, &dth);
     addf(a.facc, n, q.x, fi);
     addf(a.facc, n, q.z, fk);
     addf(a.facc, n, q.y, make_float3(-fi.x - fk.x, -fi.y - fk.y, -fi.z - fk.z));
@@ -121,9 +96,8 @@ __device__ __forceinline__ void bonded_body(const BondedArgs& a, int bid) {
     const int2 b = a.ub[r];
     const float2 pr = a.ub_prm[r];
     const float3 d = image_diff(a.pos4[b.x], a.pos4[b.y], p);
-    const float rr = sqrtf(dot(d, d));
-    const float dr = rr - pr.y;
-    const float f = rr > 0.f ? -2.f * pr.x * dr / rr : 0.f;
+    float dr;
+    const float f = bond_force(d, pr, &dr);
     addf(a.facc, n, b.x, make_float3(f * d.x, f * d.y, f * d.z));
     addf(a.facc, n, b.y, make_float3(-f * d.x, -f * d.y, -f * d.z));
     if (ENERGY) {
@@ -186,11 +160,9 @@ __device__ __forceinline__ void bonded_body(const BondedArgs& a, int bid) {
     double d[3] = {(double)ri.x - rj.x, (double)ri.y - rj.y, (double)ri.z - rj.z};
     min_image_d(d, p);
     const double r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
-    const double rr = sqrt(r2);
-    const double beta = (double)p.beta;
     const double qq = (double)ri.w * (double)rj.w;
-    const double erfv = erf(beta * rr);
-    const double f = kCC * qq * (1.1283791670955126 * beta * rr * exp(-beta * beta * r2) - erfv) / (r2 * rr);
+    double rr, erfv;
+    const double f = excl_force(r2, qq, (double)p.beta, &rr, &erfv);
     const long long fx = to_fix_d(f * d[0]), fy = to_fix_d(f * d[1]), fz = to_fix_d(f * d[2]);
     red_add(a.facc + b.x, fx);
     red_add(a.facc + n + b.x, fy);

@@ -351,6 +351,73 @@ __device__ __forceinline__ void half_kick(double* v, double3 F, double im, const
 // move it past (pointers that may alias), so that load does not wait on DRAM
 __device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
+// Forces among a rigid water's own atoms (bonds, angle, Ewald exclusion pairs) at the
+// positions its thread has just made: the first entry of the step's force accumulators,
+// stored in place of zeros.  The same values as the bonded kernel's, which took a thread
+// per term, 7 loads of atom pairs and 45 atomic adds per water in a launch of its own
+// (230,400 atoms: 17 us; 9,000 atoms: 6 us on the critical path); here the positions
+// are in registers and nothing is atomic.
+__device__ __forceinline__ void water_terms(const IntegrateArgs& a, int u, const Unit& U, const float4* x) {
+  long long f[3][3] = {};
+  const int t = a.unit_term_of[u - a.unit_term_begin];
+  if (t >= 0) {
+    const UnitTerms T = a.unit_terms[t];
+    const SysParams& p = a.p;
+    const double L[3] = {(double)p.box.x, (double)p.box.y, (double)p.box.z};
+    double d[3][3];  // atoms (0,1), (0,2), (1,2)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const float4 ra = x[k == 2 ? 1 : 0], rb = x[k == 0 ? 1 : 2];
+      d[k][0] = (double)ra.x - (double)rb.x;
+      d[k][1] = (double)ra.y - (double)rb.y;
+      d[k][2] = (double)ra.z - (double)rb.z;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) d[k][c] -= L[c] * rint(d[k][c] * a.inv_box_d[c]);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const int i = k == 2 ? 1 : 0, j = k == 0 ? 1 : 2;
+      const float3 e = make_float3((float)d[k][0], (float)d[k][1], (float)d[k][2]);
+      if (T.has >> k & 1) {
+        float dr;
+        const float g = bond_force(e, T.bond[k], &dr);
+        const long long g0 = to_fix(g * e.x), g1 = to_fix(g * e.y), g2 = to_fix(g * e.z);
+        f[i][0] += g0, f[i][1] += g1, f[i][2] += g2;
+        f[j][0] -= g0, f[j][1] -= g1, f[j][2] -= g2;
+      }
+      if (T.has >> (5 + k) & 1) {
+        const double r2 = d[k][0] * d[k][0] + d[k][1] * d[k][1] + d[k][2] * d[k][2];
+        double rr, erfv;
+        const double g = excl_force(r2, (double)x[i].w * (double)x[j].w, (double)p.beta, &rr, &erfv);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const long long gc = to_fix_d(g * d[k][c]);
+          f[i][c] += gc;
+          f[j][c] -= gc;
+        }
+      }
+    }
+    if (T.has >> 3 & 1) {
+      const bool swap = T.has >> 4 & 1;
+      // base - apex; the angle's own order of its ends
+      const float3 e1 = make_float3(-(float)d[0][0], -(float)d[0][1], -(float)d[0][2]);
+      const float3 e2 = make_float3(-(float)d[1][0], -(float)d[1][1], -(float)d[1][2]);
+      float3 fi, fk;
+      float dth;
+      angle_force(swap ? e2 : e1, swap ? e1 : e2, T.angle, &fi, &fk, &dth);
+      const float3 f1 = swap ? fk : fi, f2 = swap ? fi : fk;
+      f[1][0] += to_fix(f1.x), f[1][1] += to_fix(f1.y), f[1][2] += to_fix(f1.z);
+      f[2][0] += to_fix(f2.x), f[2][1] += to_fix(f2.y), f[2][2] += to_fix(f2.z);
+      f[0][0] += to_fix(-fi.x - fk.x), f[0][1] += to_fix(-fi.y - fk.y), f[0][2] += to_fix(-fi.z - fk.z);
+    }
+  }
+  const int n = a.p.n;
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) a.facc[(size_t)c * n + U.atom[k]] = f[k][c];
+}
+
 // NPT (Andersen barostat step with the integration units as scaling groups): the unit
 // moves rigidly with its mass centre scaled by a.lam about the origin (the box changed
 // by a.lam), and its centre-of-mass velocity is scaled by a.vfric before the kick.
@@ -359,11 +426,11 @@ __device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefe
 // to the stored float), so one pass replaces the previous step's closing launch and
 // this step's opening one with bit-identical results.
 template <bool NPT, int NA, int NC, bool SETTLE, bool CLOSE = false>
-__device__ __forceinline__ void kick_drift_body(const IntegrateArgs& a, int bid) {
+__device__ __forceinline__ void kick_drift_body(const IntegrateArgs& a, int u_begin, int u_end, int bid) {
   static_assert(!(NPT && CLOSE), "the closing pass is for constant-volume steps");
   griddep_wait();
-  const int u = a.u_begin + bid * blockDim.x + threadIdx.x;
-  if (u >= a.u_end) return;
+  const int u = u_begin + bid * blockDim.x + threadIdx.x;
+  if (u >= u_end) return;
   const Unit U = load_unit<NA, NC>(a, u);
   const int n = a.p.n;
   double r0[4][3], rn[4][3], v[4][3], im[4];
@@ -406,10 +473,12 @@ __device__ __forceinline__ void kick_drift_body(const IntegrateArgs& a, int bid)
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     if (k >= U.na) continue;
-    const int i = U.atom[k];
-    a.facc[i] = 0;
-    a.facc[n + i] = 0;
-    a.facc[2 * n + i] = 0;
+    if (!SETTLE || !a.fuse_terms) {
+      const int i = U.atom[k];
+      a.facc[i] = 0;
+      a.facc[n + i] = 0;
+      a.facc[2 * n + i] = 0;
+    }
     half_kick(v[k], F[k], im[k], a);
   }
   if (NPT) {
@@ -455,12 +524,15 @@ __device__ __forceinline__ void kick_drift_body(const IntegrateArgs& a, int bid)
       for (int c = 0; c < 3; ++c) v[k][c] = (rn[k][c] - r0[k][c]) * idt;  // v += dr/(dt TU)
   }
   bool far = false, moved = false;
+  float4 x[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     if (k >= U.na) continue;
     const int i = U.atom[k];
     const float4 np = make_float4((float)rn[k][0], (float)rn[k][1], (float)rn[k][2], q[k]);
+    x[k] = np;
     a.pos4[i] = np;
+    a.pos_drift[i] = np;
     a.vel4[i] = make_float4((float)v[k][0], (float)v[k][1], (float)v[k][2], (float)im[k]);
     a.xyzq_s[a.inv_perm[i]] = np;
     const float4 pb = a.pos_build[i];
@@ -476,15 +548,29 @@ __device__ __forceinline__ void kick_drift_body(const IntegrateArgs& a, int bid)
   const bool lead = (threadIdx.x & 31) == __ffs(am) - 1;
   if (__any_sync(am, far) && lead) *a.flag = 1;
   if (__any_sync(am, moved) && lead) *a.flag_prune = 1;
+  if constexpr (SETTLE) {
+    if (a.fuse_terms) water_terms(a, u, U, x);
+  }
 }
 
 template <bool NPT, int NA, int NC, bool SETTLE = false>
-__global__ void __launch_bounds__(128) k_kick_drift(IntegrateArgs a) { griddep_wait(); kick_drift_body<NPT, NA, NC, SETTLE>(a, blockIdx.x); }
+__global__ void __launch_bounds__(128) k_kick_drift(IntegrateArgs a) { griddep_wait(); kick_drift_body<NPT, NA, NC, SETTLE>(a, a.u_begin, a.u_end, blockIdx.x); }
 
 template <int NA, int NC, bool SETTLE>
 __global__ void __launch_bounds__(128, SETTLE ? 4 : 1) k_close_kick_drift(IntegrateArgs a) {
   griddep_wait();
-  kick_drift_body<false, NA, NC, SETTLE, true>(a, blockIdx.x);
+  kick_drift_body<false, NA, NC, SETTLE, true>(a, a.u_begin, a.u_end, blockIdx.x);
+}
+
+// free atoms (class 0) and SETTLE waters (class 1), the two classes of a solvated system
+// without other hydrogens, in one launch: the waters' blocks first, then the free atoms'
+template <bool NPT, bool CLOSE>
+__global__ void __launch_bounds__(128, 4) k_drift_free_water(const __grid_constant__ IntegrateArgs a, int nwater) {
+  griddep_wait();
+  if ((int)blockIdx.x < nwater)
+    kick_drift_body<NPT, 3, 3, true, CLOSE>(a, a.cls_begin[1], a.cls_begin[2], blockIdx.x);
+  else
+    kick_drift_body<NPT, 1, 0, false, CLOSE>(a, a.cls_begin[0], a.cls_begin[1], blockIdx.x - nwater);
 }
 
 template <int NA, int NC, bool SETTLE>
@@ -493,14 +579,14 @@ __global__ void __launch_bounds__(128, SETTLE ? 4 : 1) k_close_kick_drift_b(cons
   griddep_wait();
   const int4 t = tab[blockIdx.x];
   const IntegrateArgs a = args[t.x];
-  kick_drift_body<false, NA, NC, SETTLE, true>(a, t.y);
+  kick_drift_body<false, NA, NC, SETTLE, true>(a, a.u_begin, a.u_end, t.y);
 }
 
 template <int NA, int NC, bool SETTLE>
 __global__ void __launch_bounds__(128) k_kick_drift_b(const IntegrateArgs* __restrict__ args, const int4* __restrict__ tab) { griddep_wait();
   const int4 t = tab[blockIdx.x];
   const IntegrateArgs a = args[t.x];
-  kick_drift_body<false, NA, NC, SETTLE>(a, t.y);
+  kick_drift_body<false, NA, NC, SETTLE>(a, a.u_begin, a.u_end, t.y);
 }
 
 // Group (unit) virial terms of a barostat step, after the forces: the centre-of-mass
@@ -854,10 +940,21 @@ void for_classes(const IntegrateArgs& a0, F f) {
 
 static int unit_grid(const IntegrateArgs& a) { return (a.u_end - a.u_begin + 127) / 128; }
 
+static bool free_and_water(const IntegrateArgs& a) {
+  return a.settle && a.ncls == 2 && a.cls_na[0] == 1 && a.cls_nc[0] == 0 && a.cls_na[1] == 3 && a.cls_nc[1] == 3;
+}
+template <bool NPT, bool CLOSE>
+static void launch_free_water(const IntegrateArgs& a, cudaStream_t st) {
+  const int nw = (a.cls_begin[2] - a.cls_begin[1] + 127) / 128, nf = (a.cls_begin[1] - a.cls_begin[0] + 127) / 128;
+  launch_pdl(k_drift_free_water<NPT, CLOSE>, dim3(nw + nf), dim3(128), 0, st, a, nw);
+}
+int drift_launches(const IntegrateArgs& a) { return free_and_water(a) ? 1 : a.ncls; }
+
 // (3, 3) units go to the SETTLE instantiation when every one of them is a symmetric
 // triangle (a.settle), which keeps its registers apart from the Newton solver's
 template <bool NPT>
 static void kick_drift_classes(const IntegrateArgs& a, cudaStream_t st) {
+  if (free_and_water(a)) return launch_free_water<NPT, false>(a, st);
   for_classes(a, [&](const IntegrateArgs& x, auto na, auto nc) {
     constexpr int NA = decltype(na)::value, NC = decltype(nc)::value;
     if constexpr (NA == 3 && NC == 3) {
@@ -873,6 +970,7 @@ static void kick_drift_classes(const IntegrateArgs& a, cudaStream_t st) {
 void launch_kick_drift(const IntegrateArgs& a, cudaStream_t st) { kick_drift_classes<false>(a, st); }
 
 void launch_close_kick_drift(const IntegrateArgs& a, cudaStream_t st) {
+  if (free_and_water(a)) return launch_free_water<false, true>(a, st);
   for_classes(a, [&](const IntegrateArgs& x, auto na, auto nc) {
     constexpr int NA = decltype(na)::value, NC = decltype(nc)::value;
     if constexpr (NA == 3 && NC == 3) {

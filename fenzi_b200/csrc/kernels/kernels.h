@@ -1,5 +1,6 @@
 // Launch interfaces of the sm_100a kernels (host side of each .cu file).
 #pragma once
+#include "bonded_terms.cuh"
 #include "common.cuh"
 
 namespace fzk {
@@ -131,7 +132,20 @@ struct PmeArgs {
   int* status;
   int gather;  // gather kernel: 1 one CTA per brick, 2 one thread per atom, 0 by atoms per brick
 };
-void launch_pme(const PmeArgs& a, bool energy, cudaStream_t st);
+// cleared: launch_pme_clear has already been queued for this evaluation
+void launch_pme(const PmeArgs& a, bool energy, cudaStream_t st, bool cleared = false);
+// zeroes the charge grid (and the brick counters): needs only the last gather to be done
+void launch_pme_clear(const PmeArgs& a, cudaStream_t st);
+// PME influence tables of a box: gfac = |b(m)|^2 exp(-pi^2 f^2 / beta^2), f2 = f^2 with
+// f = m' / L, computed in FP64 and rounded once
+struct PmeTables {
+  int K[3];
+  const double* bm2[3];
+  float* gfac[3];
+  float* f2[3];
+  double box[3], beta;
+};
+void launch_pme_tables(const PmeTables& t, cudaStream_t st);
 // batched PME: the systems of one grid size share the FFT launches
 struct PmeSizeBatch {
   int N;                  // Kx = Ky (plane kernels), Kz compiled
@@ -174,6 +188,14 @@ struct IntegrateArgs {
   const int* unit_meta;     // na | nc<<4 | pairs<<8 (local a,b 2 bits each)
   const float4* unit_d;     // constraint lengths
   float4* pos4;
+  float4* pos_drift;        // copy of the drifted positions that no rebuild wraps: what PME
+                            // and the bonded kernel of a step read
+  // terms among the atoms of a SETTLE unit, evaluated where its new positions are made
+  // (fuse_terms; else the bonded kernel has them): term set of each unit, -1 none
+  const UnitTerms* unit_terms;
+  const int* unit_term_of;   // indexed by unit - unit_term_begin
+  int unit_term_begin;
+  int fuse_terms;
   float4* vel4;             // xyz velocity, w = 1/m
   long long* facc;
   float4* xyzq_s;
@@ -214,6 +236,7 @@ void launch_kick_drift_b(const ClassBatch& c, cudaStream_t st);
 void launch_kick_rattle_b(const ClassBatch& c, cudaStream_t st);
 void launch_close_kick_drift_b(const ClassBatch& c, cudaStream_t st);
 void launch_kick_drift(const IntegrateArgs& a, cudaStream_t st);
+int drift_launches(const IntegrateArgs& a);  // launches of one kick + drift pass
 // the previous step's closing kick + RATTLE and this step's kick + drift + SHAKE in one
 // pass (constant volume; bit-identical to launch_kick_rattle then launch_kick_drift)
 void launch_close_kick_drift(const IntegrateArgs& a, cudaStream_t st);

@@ -1278,20 +1278,37 @@ int pme_launches(const PmeArgs& a) {
   return (pme_mode(a) == 3 ? 1 : 5) + (use_plane_fft(a) ? 3 : 5) + 1;
 }
 
-void launch_pme(const PmeArgs& a_in, bool energy, cudaStream_t st) {
+__global__ void __launch_bounds__(128) k_pme_tables(const __grid_constant__ PmeTables t) {
+  griddep_wait();
+  int m = blockIdx.x * blockDim.x + threadIdx.x, d = 0;
+  while (d < 3 && m >= t.K[d]) m -= t.K[d++];
+  if (d == 3) return;
+  const double f = (m <= t.K[d] / 2 ? m : m - t.K[d]) / t.box[d];
+  t.f2[d][m] = (float)(f * f);
+  t.gfac[d][m] = (float)(t.bm2[d][m] * exp(-kPi * kPi * f * f / (t.beta * t.beta)));
+}
+void launch_pme_tables(const PmeTables& t, cudaStream_t st) {
+  launch_pdl(k_pme_tables, dim3((t.K[0] + t.K[1] + t.K[2] + 127) / 128), dim3(128), 0, st, t);
+}
+
+void launch_pme_clear(const PmeArgs& a, cudaStream_t st) {
+  const int nbr = a.nb[0] * a.nb[1] * a.nb[2];
+  if (pme_mode(a) != 3) launch_pdl(k_pme_zero, dim3((nbr + 255) / 256), dim3(256), 0, st, a);
+  cudaMemsetAsync(a.grid, 0, (size_t)a.K[0] * a.K[1] * a.K[2] * sizeof(float), st);
+}
+
+void launch_pme(const PmeArgs& a_in, bool energy, cudaStream_t st, bool cleared) {
   PmeArgs a = a_in;
   a.gather = pme_mode(a_in);
   const int nbr = a.nb[0] * a.nb[1] * a.nb[2];
+  if (!cleared) launch_pme_clear(a, st);
   const size_t sp = (size_t)(a.B[0] + 3) * (a.B[1] + 3) * (a.B[2] + 3) * sizeof(int);
   if (a.gather == 3) {
-    cudaMemsetAsync(a.grid, 0, (size_t)a.K[0] * a.K[1] * a.K[2] * sizeof(float), st);
     launch_pdl(k_pme_spread_atoms, dim3((4 * a.n + 255) / 256), dim3(256), 0, st, a);
   } else {
-    launch_pdl(k_pme_zero, dim3((nbr + 255) / 256), dim3(256), 0, st, a);
     launch_pdl(k_pme_bin, dim3((a.n + 255) / 256), dim3(256), 0, st, a);
     launch_pdl(k_pme_scan, dim3(1), dim3(1024), 0, st, a);
     launch_pdl(k_pme_scatter, dim3((a.n + 255) / 256), dim3(256), 0, st, a);
-    cudaMemsetAsync(a.grid, 0, (size_t)a.K[0] * a.K[1] * a.K[2] * sizeof(float), st);
     launch_pdl(k_pme_spread, dim3(nbr), dim3(256), sp, st, a);
   }
   const int Kx = a.K[0], Ky = a.K[1], Kz = a.K[2], Kxh = Kx / 2 + 1;
