@@ -179,7 +179,9 @@ static bool batched_kernels_ok(const fz_batch* b) {
   if (v && std::atoi(v) == 0) return false;
   for (const fz_system* s : b->systems) {
     const Engine* e = s->eng;
-    if (e->cond_graph || e->restraint || e->npt || !fzk::pme_batchable(e->pme_args())) return false;
+    if (e->restraint || e->npt || !fzk::pme_batchable(e->pme_args()) ||
+        !fzk::columns_scan_in_block(e->rebuild_args()))
+      return false;
   }
   return true;
 }
@@ -314,7 +316,7 @@ static fz_status build_batch_kernels(fz_batch* b) {
     FZ_CUDA(cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming));
   }
   if ((r = bk->place(b->arena, b->master))) return r;
-  bk->launches = 2 * (long long)bk->classes.size() + fzk::kRebuildBuildLaunches + fzk::kRebuildPruneLaunches +
+  bk->launches = 2 * (long long)bk->classes.size() + fzk::kRebuildLaunches +
                  1 + (bk->t.n[fzk::BT_BONDED] > 0 ? 1 : 0) + 7 + 3 * (long long)bk->sizes.size();
   b->bk = std::move(bk);
   return FZ_OK;
@@ -332,9 +334,8 @@ static void batched_step_body(fz_batch* b, cudaStream_t st, bool open = true, bo
   }
   cudaEventRecord(b->ev_fork, st);
   cudaStreamWaitEvent(b->aux, b->ev_fork, 0);
-  fzk::launch_rebuild_build_b(k.rb, k.t, st);
   fzk::launch_pme_b(k.pme, k.t, k.sizes.data(), (int)k.sizes.size(), k.spread_smem, b->aux);
-  fzk::launch_rebuild_prune_b(k.rb, k.t, st);
+  fzk::launch_rebuild_b(k.rb, k.t, st);
   fzk::launch_nonbonded_b(k.nb, k.t, k.max_ntypes, st);
   fzk::launch_bonded_b(k.bd, k.t, st);
   cudaEventRecord(b->ev_join, b->aux);
@@ -428,7 +429,6 @@ extern "C" fz_status fz_batch_step(fz_batch* b, int nsteps) {
       Engine* e = b->systems[i]->eng;
       e->step += k;
       e->launches += (long long)k * e->graph_step_launches();
-      e->graph_since_check = true;
       if (e->temp_reset_every > 0 && e->step % e->temp_reset_every == 0) {
         FZ_CUDA(cudaEventRecord(b->ev_master, b->master));
         FZ_CUDA(cudaStreamWaitEvent(e->st, b->ev_master, 0));

@@ -154,12 +154,12 @@ static fz_status autotune(Engine* e) {
   // pair-kernel CTAs per SM
   if (!fix_per_sm) {
     const int p0 = e->nb_per_sm;
-    float best = time_launches(e->st, [&] { fzk::launch_nonbonded(e->nb_args(), false, e->st); });
+    float best = time_launches(e->st, [&] { fzk::launch_nonbonded(e->nb_args(), false, e->st, true); });
     int pick = p0;
     for (int per : {4, 3, 2}) {
       if (per == p0) continue;
       set_per_sm(e, per);
-      const float t = time_launches(e->st, [&] { fzk::launch_nonbonded(e->nb_args(), false, e->st); });
+      const float t = time_launches(e->st, [&] { fzk::launch_nonbonded(e->nb_args(), false, e->st, true); });
       if (t < 0.99f * best) {
         best = t;
         pick = per;
@@ -219,18 +219,12 @@ static fz_status build_engine(fz_system* s, int device, void* stream) {
   }
   FZ_CUDA(cudaStreamCreateWithFlags(&e->st2, cudaStreamNonBlocking));
   {
-    // conditional IF nodes for the neighbour kernels inside captured steps: measured
-    // ~12 us per step slower on B200 at 230,400 atoms than the flag-checking kernels
-    // they replace, so they are off unless FZ_GRAPH_COND=1
-    const char* v = std::getenv("FZ_GRAPH_COND");
-    e->cond_graph = v && std::atoi(v) == 1;
     if (const char* c = std::getenv("FZ_GRAPH_CHUNK")) e->chunk_steps = std::max(0, std::min(1000, std::atoi(c)));
     if (const char* c = std::getenv("FZ_FUSE_CLOSE")) e->fuse_close = std::atoi(c) != 0;
   }
   FZ_CUDA(cudaEventCreateWithFlags(&e->ev_fork, cudaEventDisableTiming));
   FZ_CUDA(cudaEventCreateWithFlags(&e->ev_join, cudaEventDisableTiming));
   FZ_CUDA(cudaStreamCreateWithFlags(&e->st3, cudaStreamNonBlocking));
-  FZ_CUDA(cudaStreamCreateWithFlags(&e->st_cap, cudaStreamNonBlocking));
   FZ_CUDA(cudaEventCreateWithFlags(&e->ev_top, cudaEventDisableTiming));
   FZ_CUDA(cudaEventCreateWithFlags(&e->ev_join3, cudaEventDisableTiming));
   const int n = t.n;

@@ -124,14 +124,7 @@ struct Engine {
   int prune_split = 0;
   int outer_split = 0;
   bool use_graph = true;
-  // With cond_graph (env FZ_GRAPH_COND=1) the rebuild and prune kernels of captured
-  // steps are the bodies of two conditional IF nodes set from the device flags, else
-  // flag-checking kernels launched every step; st_cap captures the bodies.
-  bool cond_graph = false;
-  cudaStream_t st_cap = nullptr;
   cudaError_t capture_error = cudaSuccess;
-  long long seen_rb_launch = 0, seen_pr_launch = 0;  // device counters already accounted
-  bool graph_since_check = false;                     // captured steps ran since check()
   // PME runs on a second stream concurrently with the pair and bonded kernels
   cudaStream_t st2 = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -207,7 +200,6 @@ struct Engine {
     if (ev_top) cudaEventDestroy(ev_top);
     if (ev_join3) cudaEventDestroy(ev_join3);
     if (st3) cudaStreamDestroy(st3);
-    if (st_cap) cudaStreamDestroy(st_cap);
     if (st2) cudaStreamDestroy(st2);
     for (auto& x : ev)
       if (x) cudaEventDestroy(x);
@@ -287,6 +279,9 @@ struct Engine {
     // for the PME kernels of the second stream (a measurement knob)
     if (const char* v = std::getenv("FZ_NB_GRID_PER_SM")) a.grid = n_sm * std::max(1, std::min(8, std::atoi(v)));
     a.minb = nb_per_sm;
+    a.flag = flag;
+    a.flag_prune = flag_prune;
+    a.close_lists = 1;
     return a;
   }
   // step: the forces of a step, after its drift (pos_drift)
@@ -398,8 +393,9 @@ struct Engine {
   // step: after a drift whose pass has evaluated the rigid waters' own terms
   void forces(bool energies, int terms = FZ_TERM_ALL, bool step = false) {
     mark(1);
-    fzk::launch_rebuild(rebuild_args(), st);
-    launches += fzk::kRebuildBuildLaunches + fzk::kRebuildPruneLaunches;
+    const bool close = !(terms & FZ_TERM_NONBONDED);
+    fzk::launch_rebuild(rebuild_args(), st, close);
+    launches += rebuild_launches() + (close ? 1 : 0);
     mark(2);
     // PME beside the pair and bonded kernels (in line when the stages are timed)
     const bool beside = (terms & FZ_TERM_PME) && st2 && !timing;
@@ -461,88 +457,18 @@ struct Engine {
     cudaMemsetAsync(rs_acc, 0, 8 * sizeof(long long), s);
     fzk::launch_restraint(p, pos4, rs_seg, rs_mass, rs_acc, rs_inv_m[0], rs_inv_m[1], rs_dist, rs_fc, facc, s);
   }
-  // Adds to the capture on st an IF node that runs body(stream) when *dflag != 0 (or
-  // *dflag2 != 0 when given).
-  template <class F>
-  void conditional(const int* dflag, const int* dflag2, F body) {
-    cudaStreamCaptureStatus cs;
-    unsigned long long id;
-    cudaGraph_t g = nullptr;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t nd = 0;
-    cudaGraphConditionalHandle h;
-    cudaError_t e = cudaStreamGetCaptureInfo(st, &cs, &id, &g, &deps, &nd);
-    if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&h, g, 0, 0);
-    if (e != cudaSuccess) {
-      capture_error = e;
-      return;
-    }
-    fzk::launch_set_condition(h, dflag, dflag2, st);
-    e = cudaStreamGetCaptureInfo(st, &cs, &id, &g, &deps, &nd);
-    cudaGraphNodeParams np{};
-    np.type = cudaGraphNodeTypeConditional;
-    np.conditional.handle = h;
-    np.conditional.type = cudaGraphCondTypeIf;
-    np.conditional.size = 1;
-    cudaGraphNode_t node;
-    if (e == cudaSuccess) e = cudaGraphAddNode(&node, g, deps, nd, &np);
-    if (e == cudaSuccess) e = cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies);
-    if (e == cudaSuccess)
-      e = cudaStreamBeginCaptureToGraph(st_cap, np.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                        cudaStreamCaptureModeThreadLocal);
-    if (e != cudaSuccess) {
-      capture_error = e;
-      return;
-    }
-    body(st_cap);
-    cudaGraph_t out = nullptr;
-    e = cudaStreamEndCapture(st_cap, &out);
-    if (e != cudaSuccess) capture_error = e;
-  }
-  // neighbour maintenance: conditional nodes inside a capture, else flag-checking kernels
-  bool capturing_conditional() {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    return cond_graph && st_cap && cudaStreamIsCapturing(st, &cs) == cudaSuccess &&
-           cs == cudaStreamCaptureStatusActive;
-  }
-  // list rebuild when due (it wraps the positions, so it precedes every reader)
-  void rebuild_build_step() {
-    const fzk::RebuildArgs ra = rebuild_args();
-    if (capturing_conditional()) conditional(flag, nullptr, [&](cudaStream_t s) { fzk::launch_rebuild_build(ra, s); });
-    else fzk::launch_rebuild_build(ra, st);
-  }
-  // inner-list prune when due (reads the sorted positions, writes only list data)
-  void prune_step() {
-    const fzk::RebuildArgs ra = rebuild_args();
-    // a rebuild this step (flag still raised) always ends in a prune
-    if (capturing_conditional())
-      conditional(flag_prune, flag, [&](cudaStream_t s) { fzk::launch_rebuild_prune(ra, s); });
-    else fzk::launch_rebuild_prune(ra, st);
-  }
-  void rebuild_step() {
-    rebuild_build_step();
-    prune_step();
-  }
   // kernels one captured step launches
   long long graph_step_launches() const {
-    return fzk::drift_launches(int_args()) + ncls +
-           (cond_graph ? 2 : fzk::kRebuildBuildLaunches + fzk::kRebuildPruneLaunches) + 1 + bonded_step_launches() +
+    return fzk::drift_launches(int_args()) + ncls + rebuild_launches() + 1 + bonded_step_launches() +
            fzk::pme_launches(pme_args()) + (restraint ? 2 : 0);
+  }
+  int rebuild_launches() const {
+    return fzk::kRebuildLaunches + (fzk::columns_scan_in_block(rebuild_args()) ? 0 : 1);
   }
   int bonded_step_launches() const {
     return (nbond_step + nangle_step + nub + ndihe + nimpr + nexcl_step + n14 > 0) ? 1 : 0;
   }
   int bonded_launches() const { return (nbond + nangle + nub + ndihe + nimpr + nexcl + n14 > 0) ? 1 : 0; }
-  // launches of the conditional bodies (per rebuild and per prune) since the last
-  // call, from the device counters; called after a synchronisation
-  void account_conditional(const int* cnt) {
-    if (cond_graph && graph_since_check)
-      launches += fzk::kRebuildBuildLaunches * (cnt[fzk::CNT_REBUILDS] - seen_rb_launch) +
-                  fzk::kRebuildPruneLaunches * (cnt[fzk::CNT_PRUNES] - seen_pr_launch);
-    graph_since_check = false;
-    seen_rb_launch = cnt[fzk::CNT_REBUILDS];
-    seen_pr_launch = cnt[fzk::CNT_PRUNES];
-  }
   // One MD step.  open: the step starts with its own kick + drift pass (else the
   // previous step left its closing kick + RATTLE to this step's first pass); close: the
   // step ends with the kick + RATTLE pass (else the next step's first pass does it).
@@ -575,7 +501,7 @@ struct Engine {
       fzk::launch_bonded(bonded_args(true), false, st3);
       cudaEventRecord(ev_join3, st3);
     }
-    rebuild_step();
+    fzk::launch_rebuild(rebuild_args(), st, false);
     fzk::launch_nonbonded(nb_args(), false, st);
     if (restraint) restraint_forces(st);
     if (bonded) cudaStreamWaitEvent(st, ev_join3, 0);
@@ -599,7 +525,6 @@ struct Engine {
     }
     FZ_CUDA(cudaGraphLaunch(step_exec, st));
     launches += graph_step_launches();
-    graph_since_check = true;
     return FZ_OK;
   }
   // chunk_steps steps in one graph launch (captured on first use)
@@ -620,7 +545,6 @@ struct Engine {
     }
     FZ_CUDA(cudaGraphLaunch(chunk_exec, st));
     launches += (long long)chunk_steps * graph_step_launches() - (fuse_close ? (long long)(chunk_steps - 1) * ncls : 0);
-    graph_since_check = true;
     return FZ_OK;
   }
   void drop_graph() {
@@ -644,7 +568,6 @@ struct Engine {
     FZ_CUDA(cudaMemcpyAsync(b, energy, sizeof(Readback), cudaMemcpyDeviceToHost, st));
     FZ_CUDA(cudaStreamSynchronize(st));
     FZ_CUDA(cudaGetLastError());
-    account_conditional(b->counters);
     return status_of(b->status);
   }
   fz_status check() {

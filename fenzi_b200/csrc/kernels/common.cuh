@@ -90,6 +90,21 @@ inline void launch_pdl(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cuda
   cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
 }
 
+// list counters of a system (kernels.h names them all)
+enum : int {
+  CNT_TILES = 0, CNT_MASKS, CNT_SLOTS, CNT_REBUILDS, CNT_PRUNES, CNT_WORK, CNT_ITEMS, CNT_COUNT = 8
+};
+// end of the neighbour launches of a step: counts what was done, lowers the flags
+__device__ __forceinline__ void lists_close(int* flag, int* flag_prune, int* counters) {
+  const int build = *flag, prune = *flag_prune;
+  if (build) counters[CNT_REBUILDS] += 1;
+  if (build || prune) {
+    counters[CNT_PRUNES] += 1;
+    *flag = 0;
+    *flag_prune = 0;
+  }
+}
+
 __device__ __forceinline__ long long to_fix(float f) { return __float2ll_rn(f * kFixF); }
 __device__ __forceinline__ long long to_fix_d(double f) { return __double2ll_rn(f * kFixFd); }
 

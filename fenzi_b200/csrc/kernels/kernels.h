@@ -8,12 +8,8 @@ namespace fzk {
 constexpr int kColCap = 4096;  // atoms per column sorted in shared memory
 constexpr int kWarpsPerCta = 8;  // warps of a pair-kernel CTA
 constexpr int kNbBatchCtasPerSm = 4;  // CTAs per SM the batched pair kernel is built and launched for
-enum : int {
-  CNT_TILES = 0, CNT_MASKS, CNT_SLOTS, CNT_REBUILDS, CNT_PRUNES, CNT_WORK, CNT_ITEMS, CNT_COUNT = 8
-};
 // kernels each launcher issues (the step's launch count)
-constexpr int kRebuildBuildLaunches = 6;  // launch_rebuild_build
-constexpr int kRebuildPruneLaunches = 3;  // launch_rebuild_prune
+constexpr int kRebuildLaunches = 6;  // launch_rebuild without its close, launch_rebuild_b
 
 // Batched launches: one kernel launch covers many systems.  A block table holds one
 // int4 per launched block: (index into the launch's argument array, the block's index
@@ -76,15 +72,11 @@ struct RebuildArgs {
 };
 // whether the CTA-per-block prune's shared memory (kNG x ocap entries) fits
 bool prune_split_fits(int ocap);
-void launch_rebuild(const RebuildArgs& a, cudaStream_t st);
-// the two halves of launch_rebuild: the outer-list build (flag) and the prune (flag_prune)
-void launch_rebuild_build(const RebuildArgs& a, cudaStream_t st);
-void launch_rebuild_prune(const RebuildArgs& a, cudaStream_t st);
-void launch_rebuild_build_b(const RebuildArgs* args, const BatchTables& t, cudaStream_t st);
-void launch_rebuild_prune_b(const RebuildArgs* args, const BatchTables& t, cudaStream_t st);
-// one-thread kernel: graph conditional value = (*flag != 0)
-// IF-node value = (*flag || (flag2 && *flag2))
-void launch_set_condition(cudaGraphConditionalHandle h, const int* flag, const int* flag2, cudaStream_t st);
+bool columns_scan_in_block(const RebuildArgs& a);
+// outer-list build (when flag is up) and prune (when either flag is); close: lower the
+// flags too (else the pair kernel that follows does: NonbondedArgs::close_lists)
+void launch_rebuild(const RebuildArgs& a, cudaStream_t st, bool close = true);
+void launch_rebuild_b(const RebuildArgs* args, const BatchTables& t, cudaStream_t st);
 
 struct NonbondedArgs {
   SysParams p;
@@ -105,8 +97,11 @@ struct NonbondedArgs {
   int ocap;
   int grid;
   int minb;  // CTAs per SM the kernel is built for (3 or 4)
+  int close_lists;  // the first block closes the neighbour launches it follows
+  int *flag, *flag_prune;
 };
-void launch_nonbonded(const NonbondedArgs& a, bool energy, cudaStream_t st);
+// zero_work: the item counter is zeroed first (a launch that follows no launch_rebuild)
+void launch_nonbonded(const NonbondedArgs& a, bool energy, cudaStream_t st, bool zero_work = false);
 void launch_nonbonded_b(const NonbondedArgs* args, const BatchTables& t, int max_ntypes, cudaStream_t st);
 
 struct PmeArgs {

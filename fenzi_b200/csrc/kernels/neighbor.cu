@@ -15,6 +15,9 @@
 
 namespace fzk {
 
+// columns whose sizes one block scans in shared memory (16 KB)
+constexpr int kScanCols = 4096;
+
 // wrap positions into [-L/2, L/2), record build positions, bin into columns
 __device__ __forceinline__ void rb_bin_body(const RebuildArgs& A, int bid, int nbid) {
   griddep_wait();
@@ -26,6 +29,16 @@ __device__ __forceinline__ void rb_bin_body(const RebuildArgs& A, int bid, int n
   int* col_count = A.col_count;
   int* status = A.status;
 
+  // first launch of the chain: opens the list counters of a prune (a rebuild ends in
+  // one) and the pair kernel's item counter
+  if (bid == 0 && threadIdx.x == 0) {
+    A.counters[CNT_WORK] = 0;
+    if (*flag || *A.flag_prune) {
+      A.counters[CNT_MASKS] = 0;
+      A.counters[CNT_TILES] = 0;
+      A.counters[CNT_ITEMS] = 0;
+    }
+  }
   if (!*flag) return;
   const int a = bid * blockDim.x + threadIdx.x;
   if (a >= p.n) return;
@@ -61,24 +74,17 @@ __global__ void k_rb_bin_b(const RebuildArgs* __restrict__ args, const int4* __r
 }
 
 
-// exclusive scan of the 32-padded column sizes (one block)
-__device__ __forceinline__ void rb_scan_body(const RebuildArgs& A, int bid, int nbid) {
-  griddep_wait();
-  const SysParams p = A.p;
-  const int* __restrict__ flag = A.flag;
-  const int* __restrict__ col_count = A.col_count;
-  int* col_start = A.col_start;
-  const int ncol = A.p.ncol[0] * A.p.ncol[1];
-  int* counters = A.counters;
-  int* status = A.status;
-
-  if (!*flag) return;
-  __shared__ int part[1024];
+// exclusive scan of the 32-padded column sizes by one block: start[c] for every column;
+// `publish`: this block also writes what the later launches read
+__device__ __forceinline__ void rb_scan(const RebuildArgs& A, int* start, bool publish) {
+  const SysParams& p = A.p;
+  const int ncol = p.ncol[0] * p.ncol[1];
+  __shared__ int part[256];
   const int t = threadIdx.x, nt = blockDim.x;
   const int per = (ncol + nt - 1) / nt;
   const int b = t * per, e = min(ncol, b + per);
   int s = 0;
-  for (int c = b; c < e; ++c) s += (col_count[c] + 31) & ~31;
+  for (int c = b; c < e; ++c) s += (A.col_count[c] + 31) & ~31;
   part[t] = s;
   __syncthreads();
   for (int o = 1; o < nt; o <<= 1) {
@@ -89,54 +95,57 @@ __device__ __forceinline__ void rb_scan_body(const RebuildArgs& A, int bid, int 
   }
   int run = part[t] - s;
   for (int c = b; c < e; ++c) {
-    col_start[c] = run;
-    run += (col_count[c] + 31) & ~31;
+    start[c] = run;
+    if (publish && start != A.col_start) A.col_start[c] = run;
+    run += (A.col_count[c] + 31) & ~31;
   }
-  if (t == nt - 1) {
+  if (publish && t == nt - 1) {
     const int used = part[t];
     // the last 32 slots are reserved for the permanent dummy block
-    if (used > p.nslots - 32) atomicOr(status, ST_SLOT_OVERFLOW);
-    counters[CNT_SLOTS] = min(used, p.nslots - 32);
-    col_start[ncol] = min(used, p.nslots - 32);
+    if (used > p.nslots - 32) atomicOr(A.status, ST_SLOT_OVERFLOW);
+    A.counters[CNT_SLOTS] = min(used, p.nslots - 32);
+    A.col_start[ncol] = min(used, p.nslots - 32);
   }
+  __syncthreads();
 }
 
-__global__ void k_rb_scan(RebuildArgs a) { griddep_wait(); rb_scan_body(a, blockIdx.x, gridDim.x); }
-__global__ void k_rb_scan_b(const RebuildArgs* __restrict__ args, const int4* __restrict__ tab) { griddep_wait();
-  const int4 t = tab[blockIdx.x];
-  const RebuildArgs a = args[t.x];
-  rb_scan_body(a, t.y, t.z);
+// systems of more columns than a block scans in shared memory: a launch of its own
+__global__ void __launch_bounds__(256) k_rb_scan(RebuildArgs a) {
+  griddep_wait();
+  if (!*a.flag) return;
+  rb_scan(a, a.col_start, true);
 }
 
-
+// Atoms into their columns.  Every block scans the column sizes itself (a few hundred
+// sums from L2) instead of waiting for a launch of one block that does; SCANNED: the
+// scan has been a launch (more than kScanCols columns).
+template <bool SCANNED>
 __device__ __forceinline__ void rb_scatter_body(const RebuildArgs& A, int bid, int nbid) {
   griddep_wait();
-  const SysParams p = A.p;
-  const int* __restrict__ flag = A.flag;
-  const int* __restrict__ col_of = A.col_of;
-  const int* __restrict__ col_start = A.col_start;
-  int* col_cursor = A.col_cursor;
-  int* col_tmp = A.col_tmp;
-
-  if (!*flag) return;
+  const SysParams& p = A.p;
+  if (!*A.flag) return;
+  __shared__ int start_s[SCANNED ? 1 : kScanCols];
+  if (!SCANNED) rb_scan(A, start_s, bid == 0);
+  const int* start = SCANNED ? A.col_start : start_s;
   const int a = bid * blockDim.x + threadIdx.x;
   if (a >= p.n) return;
-  const int c = col_of[a];
+  const int c = A.col_of[a];
   const unsigned peers = __match_any_sync(__activemask(), c);
   const int leader = __ffs(peers) - 1;
   int base = 0;
-  if ((threadIdx.x & 31) == leader) base = atomicAdd(&col_cursor[c], __popc(peers));
+  if ((threadIdx.x & 31) == leader) base = atomicAdd(&A.col_cursor[c], __popc(peers));
   base = __shfl_sync(peers, base, leader);
   const int k = base + __popc(peers & ((1u << (threadIdx.x & 31)) - 1u));
-  const int s = col_start[c] + k;
-  if (s < p.nslots - 32) col_tmp[s] = a;
+  const int s = start[c] + k;
+  if (s < p.nslots - 32) A.col_tmp[s] = a;
 }
 
-__global__ void k_rb_scatter(RebuildArgs a) { griddep_wait(); rb_scatter_body(a, blockIdx.x, gridDim.x); }
-__global__ void k_rb_scatter_b(const RebuildArgs* __restrict__ args, const int4* __restrict__ tab) { griddep_wait();
+template <bool SCANNED>
+__global__ void __launch_bounds__(256) k_rb_scatter(RebuildArgs a) { griddep_wait(); rb_scatter_body<SCANNED>(a, blockIdx.x, gridDim.x); }
+__global__ void __launch_bounds__(256) k_rb_scatter_b(const RebuildArgs* __restrict__ args, const int4* __restrict__ tab) { griddep_wait();
   const int4 t = tab[blockIdx.x];
   const RebuildArgs a = args[t.x];
-  rb_scatter_body(a, t.y, t.z);
+  rb_scatter_body<false>(a, t.y, t.z);
 }
 
 
@@ -451,33 +460,6 @@ __global__ void k_rb_slots_b(const RebuildArgs* __restrict__ args, const int4* _
 }
 
 
-// Closes a rebuild (counts it, lowers its flag, raises the prune flag: a new outer list
-// always gets a fresh inner list) and opens a prune (zeroes the list counters).
-__device__ __forceinline__ void prune_begin_body(const RebuildArgs& A, int bid, int nbid) {
-  griddep_wait();
-  int* flag = A.flag;
-  int* flag_prune = A.flag_prune;
-  int* counters = A.counters;
-
-  if (*flag) {
-    counters[CNT_REBUILDS] += 1;
-    *flag = 0;
-    *flag_prune = 1;
-  }
-  if (!*flag_prune) return;
-  counters[CNT_MASKS] = 0;
-  counters[CNT_TILES] = 0;
-  counters[CNT_ITEMS] = 0;
-}
-
-__global__ void k_prune_begin(RebuildArgs a) { griddep_wait(); prune_begin_body(a, blockIdx.x, gridDim.x); }
-__global__ void k_prune_begin_b(const RebuildArgs* __restrict__ args, const int4* __restrict__ tab) { griddep_wait();
-  const int4 t = tab[blockIdx.x];
-  const RebuildArgs a = args[t.x];
-  prune_begin_body(a, t.y, t.z);
-}
-
-
 // Exclusion masks of one tile (this lane holding j entry je): the lane walks the
 // excluded partners (1-2, 1-3, 1-4) of its own j slot (xs/xn: partner slots per slot,
 // written at every rebuild) and, for each partner sitting in i-block I, sets bit
@@ -609,7 +591,7 @@ __device__ __forceinline__ void prune_body(const RebuildArgs& A, int bid, int nb
   int chunk = A.chunk;
   int* status = A.status;
 
-  if (!*flag_prune) return;
+  if (!*flag_prune && !*A.flag) return;  // a rebuild always ends in a prune
   __shared__ float4 iA_all[8][16], iB_all[8][16];
   __shared__ uint32_t buf_all[8][kNG][64];
   __shared__ uint32_t msk_all[8][32];
@@ -762,7 +744,7 @@ constexpr int kPruneWarps = 8;
 __device__ __forceinline__ void prune_split_body(const RebuildArgs& A, int I) {
   griddep_wait();
   const SysParams p = A.p;
-  if (!*A.flag_prune) return;
+  if (!*A.flag_prune && !*A.flag) return;
   const int nblk = A.counters[CNT_SLOTS] >> 5;
   if (I >= nblk) return;
   extern __shared__ uint32_t kept[];  // [kNG][ocap]
@@ -889,68 +871,40 @@ __global__ void __launch_bounds__(kPruneWarps * 32) k_prune_split(RebuildArgs a)
   prune_split_body(a, blockIdx.x);
 }
 
-__device__ __forceinline__ void prune_end_body(const RebuildArgs& A, int bid, int nbid) {
+// Closes the chain: counts what was done and lowers the flags.  Inside a step or a force
+// call the pair kernel's first block does this (NonbondedArgs::close_lists).
+__global__ void k_lists_close(RebuildArgs a) {
   griddep_wait();
-  int* flag_prune = A.flag_prune;
-  int* counters = A.counters;
-
-  counters[CNT_WORK] = 0;  // the pair kernel's item counter (it always follows)
-  if (!*flag_prune) return;
-  counters[CNT_PRUNES] += 1;
-  *flag_prune = 0;
-}
-
-__global__ void k_prune_end(RebuildArgs a) { griddep_wait(); prune_end_body(a, blockIdx.x, gridDim.x); }
-__global__ void k_prune_end_b(const RebuildArgs* __restrict__ args, const int4* __restrict__ tab) { griddep_wait();
-  const int4 t = tab[blockIdx.x];
-  const RebuildArgs a = args[t.x];
-  prune_end_body(a, t.y, t.z);
-}
-
-
-// sets a graph conditional node's value from a device flag (the neighbour kernels run
-// inside an IF node only when their flag is raised)
-__global__ void k_set_condition(cudaGraphConditionalHandle h, const int* __restrict__ flag,
-                                const int* __restrict__ flag2) { griddep_wait();
-  cudaGraphSetConditional(h, (*flag != 0 || (flag2 && *flag2 != 0)) ? 1u : 0u);
+  lists_close(a.flag, a.flag_prune, a.counters);
 }
 
 // ------------------------------------------------------------------ launchers
-void launch_set_condition(cudaGraphConditionalHandle h, const int* flag, const int* flag2, cudaStream_t st) {
-  k_set_condition<<<1, 1, 0, st>>>(h, flag, flag2);
-}
+bool columns_scan_in_block(const RebuildArgs& a) { return a.p.ncol[0] * a.p.ncol[1] <= kScanCols; }
 
-void launch_rebuild(const RebuildArgs& a, cudaStream_t st) {
-  launch_rebuild_build(a, st);
-  launch_rebuild_prune(a, st);
-}
-
-void launch_rebuild_build(const RebuildArgs& a, cudaStream_t st) {
+void launch_rebuild(const RebuildArgs& a, cudaStream_t st, bool close) {
   const SysParams& p = a.p;
   const int ncol = p.ncol[0] * p.ncol[1];
   const int maxblk = (p.nslots) / 32;
   launch_pdl(k_rb_bin, dim3((p.n + 255) / 256), dim3(256), 0, st, a);
-  launch_pdl(k_rb_scan, dim3(1), dim3(1024), 0, st, a);
-  launch_pdl(k_rb_scatter, dim3((p.n + 255) / 256), dim3(256), 0, st, a);
+  if (columns_scan_in_block(a)) {
+    launch_pdl(k_rb_scatter<false>, dim3((p.n + 255) / 256), dim3(256), 0, st, a);
+  } else {
+    launch_pdl(k_rb_scan, dim3(1), dim3(256), 0, st, a);
+    launch_pdl(k_rb_scatter<true>, dim3((p.n + 255) / 256), dim3(256), 0, st, a);
+  }
   launch_pdl(k_rb_colsort, dim3(ncol), dim3(256), kColCap * sizeof(unsigned long long), st, a);
   launch_pdl(k_rb_slots, dim3((p.nslots + 255) / 256), dim3(256), 0, st, a);
   if (a.outer_split)
     launch_pdl(k_rb_outer_split, dim3(maxblk), dim3(kOuterWarps * 32), 0, st, a);
   else
     launch_pdl(k_rb_outer, dim3((maxblk + 7) / 8), dim3(256), 0, st, a);
-}
-
-void launch_rebuild_prune(const RebuildArgs& a, cudaStream_t st) {
-  const SysParams& p = a.p;
-  const int maxblk = (p.nslots) / 32;
-  launch_pdl(k_prune_begin, dim3(1), dim3(1), 0, st, a);
   if (a.prune_split) {
     const size_t smem = (size_t)kNG * a.ocap * sizeof(uint32_t);
     launch_pdl(k_prune_split, dim3(maxblk), dim3(kPruneWarps * 32), smem, st, a);
   } else {
     launch_pdl(k_prune, dim3((maxblk + 7) / 8), dim3(256), 0, st, a);
   }
-  launch_pdl(k_prune_end, dim3(1), dim3(1), 0, st, a);
+  if (close) launch_pdl(k_lists_close, dim3(1), dim3(1), 0, st, a);
 }
 
 // (sets the kernel's dynamic shared-memory limit on the current device)
@@ -975,19 +929,13 @@ void rebuild_grids(const RebuildArgs& a, int* g6) {
   g6[3] = (maxblk + 7) / 8;           // outer, prune
 }
 
-void launch_rebuild_build_b(const RebuildArgs* args, const BatchTables& t, cudaStream_t st) {
+void launch_rebuild_b(const RebuildArgs* args, const BatchTables& t, cudaStream_t st) {
   launch_pdl(k_rb_bin_b, dim3(t.n[BT_ATOMS256]), dim3(256), 0, st, args, t.tab[BT_ATOMS256]);
-  launch_pdl(k_rb_scan_b, dim3(t.n[BT_ONE]), dim3(1024), 0, st, args, t.tab[BT_ONE]);
   launch_pdl(k_rb_scatter_b, dim3(t.n[BT_ATOMS256]), dim3(256), 0, st, args, t.tab[BT_ATOMS256]);
   launch_pdl(k_rb_colsort_b, dim3(t.n[BT_COLUMNS]), dim3(256), kColCap * sizeof(unsigned long long), st, args, t.tab[BT_COLUMNS]);
   launch_pdl(k_rb_slots_b, dim3(t.n[BT_SLOTS256]), dim3(256), 0, st, args, t.tab[BT_SLOTS256]);
   launch_pdl(k_rb_outer_b, dim3(t.n[BT_BLOCKS8]), dim3(256), 0, st, args, t.tab[BT_BLOCKS8]);
-}
-
-void launch_rebuild_prune_b(const RebuildArgs* args, const BatchTables& t, cudaStream_t st) {
-  launch_pdl(k_prune_begin_b, dim3(t.n[BT_ONE]), dim3(1), 0, st, args, t.tab[BT_ONE]);
   launch_pdl(k_prune_b, dim3(t.n[BT_BLOCKS8]), dim3(256), 0, st, args, t.tab[BT_BLOCKS8]);
-  launch_pdl(k_prune_end_b, dim3(t.n[BT_ONE]), dim3(1), 0, st, args, t.tab[BT_ONE]);
 }
 
 }  // namespace fzk

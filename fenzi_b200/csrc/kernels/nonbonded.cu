@@ -202,8 +202,9 @@ __device__ __forceinline__ void nonbonded_body(const SysParams& p, const PairCon
     const int* __restrict__ perm, const uint32_t* __restrict__ inner, const int* __restrict__ inner_nt,
     const int* __restrict__ inner_m, const uint32_t* __restrict__ dmask, const uint32_t* __restrict__ masks,
     int* __restrict__ counters, const int2* __restrict__ items, int chunk, const float2* __restrict__ ljtab,
-    long long* __restrict__ facc, long long* __restrict__ energy, int ocap) {
+    long long* __restrict__ facc, long long* __restrict__ energy, int ocap, int* closing, int* closing_prune) {
   griddep_wait();
+  if (closing && threadIdx.x == 0) lists_close(closing, closing_prune, counters);
   extern __shared__ float2 lj[];
   __shared__ float4 jx_all[kWarps][64];
   __shared__ int jt_all[kWarps][64];
@@ -300,9 +301,9 @@ __global__ void __launch_bounds__(256, MINB)
                 const int* __restrict__ inner_m, const uint32_t* __restrict__ dmask,
                 const uint32_t* __restrict__ masks, int* __restrict__ counters, const int2* __restrict__ items,
                 int chunk, const float2* __restrict__ ljtab, long long* __restrict__ facc,
-                long long* __restrict__ energy, int ocap) { griddep_wait();
+                long long* __restrict__ energy, int ocap, int* flag, int* flag_prune) { griddep_wait();
   nonbonded_body<ENERGY>(p, c, xyzq, typ, perm, inner, inner_nt, inner_m, dmask, masks, counters, items, chunk, ljtab,
-                         facc, energy, ocap);
+                         facc, energy, ocap, blockIdx.x == 0 ? flag : nullptr, flag_prune);
 }
 
 // batched: every CTA serves one system's work queue (force variant only)
@@ -312,22 +313,23 @@ __global__ void __launch_bounds__(256, kNbBatchCtasPerSm) k_nonbonded_b(const No
   const NonbondedArgs a = args[t.x];
   const PairConst c = pair_const(a.p);
   nonbonded_body<false>(a.p, c, a.xyzq_s, a.typ_s, a.perm, a.inner, a.inner_nt, a.inner_m, a.dmask, a.masks,
-                        a.counters, a.items, a.chunk, a.ljtab, a.facc, a.energy, a.ocap);
+                        a.counters, a.items, a.chunk, a.ljtab, a.facc, a.energy, a.ocap,
+                        t.y == 0 ? a.flag : nullptr, a.flag_prune);
 }
 
-void launch_nonbonded(const NonbondedArgs& a, bool energy, cudaStream_t st) {
+void launch_nonbonded(const NonbondedArgs& a, bool energy, cudaStream_t st, bool zero_work) {
   const int nt1 = a.p.ntypes + 1;
   const size_t smem = (size_t)nt1 * nt1 * sizeof(float2);
   const PairConst c = pair_const(a.p);
-  cudaMemsetAsync(a.counters + CNT_WORK, 0, sizeof(int), st);
+  if (zero_work) cudaMemsetAsync(a.counters + CNT_WORK, 0, sizeof(int), st);
   // 3 CTAs per SM fit 80 registers a thread; the 4-CTA build is held to 64
   auto k = energy ? (a.minb >= 4 ? k_nonbonded<true, 4> : k_nonbonded<true, 3>)
                   : (a.minb >= 4 ? k_nonbonded<false, 4> : k_nonbonded<false, 3>);
   launch_pdl(k, dim3(a.grid), dim3(kWarps * 32), smem, st, a.p, c, a.xyzq_s, a.typ_s, a.perm, a.inner, a.inner_nt, a.inner_m, a.dmask,
-                                       a.masks, a.counters, a.items, a.chunk, a.ljtab, a.facc, a.energy, a.ocap);
+                                       a.masks, a.counters, a.items, a.chunk, a.ljtab, a.facc, a.energy, a.ocap,
+                                       a.close_lists ? a.flag : nullptr, a.flag_prune);
 }
 
-// the work counters are zeroed by the prune's last kernel every step in batched steps
 void launch_nonbonded_b(const NonbondedArgs* args, const BatchTables& t, int max_ntypes, cudaStream_t st) {
   const size_t smem = (size_t)(max_ntypes + 1) * (max_ntypes + 1) * sizeof(float2);
   launch_pdl(k_nonbonded_b, dim3(t.n[BT_NB]), dim3(kWarps * 32), smem, st, args, t.tab[BT_NB]);
