@@ -1,14 +1,15 @@
 // Real-space nonbonded pair kernel: CHARMM LJ with the switch from ron to rc plus
 // erfc real-space Ewald, the functional form of nonbondforce (src/nonbonded_forces.cu:114-245).
 //
-// B200 design: one warp per tile (32 i-atoms of a sorted block x 32 j-atoms of the
+// B200 design: one warp per tile (16 i-atoms of half a sorted block x 32 j-atoms of the
 // pair list), each pair evaluated once (Newton's third law).  i data live in
-// registers; the tile's j data (x, y, z, q, LJ type, periodic image applied) are
-// staged once into a doubled 64-entry shared-memory ring, so at step k lane l reads
-// j = l + k with a constant-offset load and no wrap arithmetic; only the j force
-// accumulator rotates through the warp (3 shuffles per pair step).  Tiles without
+// registers, two atoms a lane; the tile's j data (x, y, z, q, LJ type, periodic image
+// applied) are staged once into a doubled shared-memory ring, so at step k a lane reads
+// its j with a constant-offset load and no wrap arithmetic; only the j force
+// accumulator rotates through the lanes (3 shuffles per two pairs).  Tiles without
 // excluded pairs (the large majority) run a mask-free loop.  The kernel is FP32-issue
-// bound, so every pair-step instruction counts:
+// bound, so every pair-step instruction counts (230,400 atoms: 246 M warp instructions
+// and 280 us a launch with one i atom a lane, 232 M and 262 us with two):
 //   erfc(x) = t P(t) exp(-x^2), t = 1/(1 + p x)  (Abramowitz & Stegun, Handbook of
 //     Mathematical Functions (1964) eq. 7.1.26, |error| <= 1.5e-7), with exp2 and the
 //     constants pre-scaled so exp(-x^2) is one multiply and one MUFU.EX2;
@@ -91,12 +92,11 @@ __device__ __forceinline__ float pair_force(const PairConst& c, float r2, float 
   const float s2 = ls.y * r2inv;
   const float s6 = s2 * s2 * s2;
   const float a6 = ls.x * s6;
-  const float b6 = a6 * s6;
+  const float e6 = fmaf(a6, s6, -a6);  // b6 - a6
   const float t = __saturatef(fmaf(r2, c.sw_a, c.sw_b));
   const float t2 = t * t;
   const float sw = fmaf(-t2, fmaf(-2.f, t, 3.f), 1.f);
-  const float e6 = b6 - a6;
-  const float h = fmaf(fmaf(2.f, b6, -a6), sw, qex * fmaf(poly, rinv, c.c2b));
+  const float h = fmaf(fmaf(2.f, e6, a6), sw, qex * fmaf(poly, rinv, c.c2b));
   const float fr = fmaf(h, r2inv, e6 * ((t - t2) * c.dsw_k));
   if (ENERGY) {
     ev += ok ? e6 * sw * (1.f / 6.f) : 0.f;
@@ -106,19 +106,77 @@ __device__ __forceinline__ float pair_force(const PairConst& c, float r2, float 
 }
 
 // One tile of kIG i atoms x 32 j entries (xj, tyj: this lane's entry, loaded by the
-// caller one tile ahead).  Lane = h * kIG + il holds i atom il of the
-// group and works on segment h of the j entries (kIG of them); the tile's j data
+// caller one tile ahead).  Lane = seg * kIL + il holds i atoms il and il + kIL of the
+// group and works on segment seg of the j entries (kIL of them); the tile's j data
 // (image shift applied) are staged in this warp's shared ring, doubled within each
-// segment, so at step k lane il reads entry h * kIG + (il + k) % kIG at a constant
-// offset; the i force stays in registers, each j force accumulator rotates through
-// its segment (3 width-kIG shuffles per step) and is back on the lane that loaded the
-// entry after kIG steps.  excl: bit e set when entry e is excluded for this lane's i.
+// segment, so at step k lane il reads entry seg * kIL + (il + k) % kIL at a constant
+// offset for both of its i atoms; the i forces stay in registers, each j force
+// accumulator takes both pairs of the step, then rotates through its segment (3
+// width-kIL shuffles per two pairs) and is back on the lane that loaded the entry
+// after kIL steps.  Two i atoms a lane against one: per pair half the ring loads and
+// half the shuffles, and two independent chains of arithmetic.
+// ex0, ex1: bit e set when entry e is excluded for i atom il / il + kIL.
+constexpr int kIL = kIG / 2;        // lanes across the i atoms
+constexpr int kSeg = 32 / kIL;      // j segments of a tile
+constexpr int kTyStride = 3 * kIL;  // ring of j types: segments on different banks
+
 template <bool ENERGY>
-__device__ __forceinline__ void run_tile(const PairConst& c, const SysParams& p, const float4& xi, float qi,
-                                         const float2* ljrow, uint32_t je, uint32_t excl, float4 xj, int tyj,
-                                         float4* jx, int* jt, const int* __restrict__ perm,
-                                         long long* __restrict__ facc, int lane, int src, float& fix, float& fiy,
-                                         float& fiz, float& ev, float& ee, float* vir) {
+__device__ __forceinline__ float pair_step(const PairConst& c, const float4& xi, float qi, const char* ljrow,
+                                           const float4& b, int tyb, bool allowed, float& dx, float& dy, float& dz,
+                                           float& fx, float& fy, float& fz, float& ev, float& ee, float* vir) {
+  dx = xi.x - b.x;
+  dy = xi.y - b.y;
+  dz = xi.z - b.z;
+  const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+  const float2 ls = *reinterpret_cast<const float2*>(ljrow + tyb);
+  const float fr = pair_force<ENERGY>(c, r2, qi * b.w, ls, r2 < c.rc2 && allowed, ev, ee);
+  if (ENERGY) {
+    vir[0] = fmaf(fr * dx, dx, vir[0]);
+    vir[1] = fmaf(fr * dy, dy, vir[1]);
+    vir[2] = fmaf(fr * dz, dz, vir[2]);
+  }
+  fx = fmaf(fr, dx, fx);
+  fy = fmaf(fr, dy, fy);
+  fz = fmaf(fr, dz, fz);
+  return fr;
+}
+
+template <bool ENERGY, bool MASKED>
+__device__ __forceinline__ void tile_steps(const PairConst& c, const float4& x0, const float4& x1, float q0, float q1,
+                                           const char* lj0, const char* lj1, uint32_t m0, uint32_t m1,
+                                           const float4* jxl, const int* jtl, int src, float* f0, float* f1, float& ev,
+                                           float& ee, float* vir, float& fjx, float& fjy, float& fjz) {
+  // the common loop whole, the rare one rolled: the two must stay in the instruction cache
+  // together (both whole: 47 % of the stalls were instruction fetches, 1.4 times the time)
+  constexpr int kUnroll = MASKED ? 1 : kIL;
+#pragma unroll kUnroll
+  for (int k = 0; k < kIL; ++k) {
+    const float4 b = jxl[k];
+    const int ty = jtl[k];
+    float dx, dy, dz, ex, ey, ez;
+    const float fa = pair_step<ENERGY>(c, x0, q0, lj0, b, ty, !MASKED || !((m0 >> k) & 1u), dx, dy, dz, f0[0], f0[1],
+                                       f0[2], ev, ee, vir);
+    const float fb = pair_step<ENERGY>(c, x1, q1, lj1, b, ty, !MASKED || !((m1 >> k) & 1u), ex, ey, ez, f1[0], f1[1],
+                                       f1[2], ev, ee, vir);
+    fjx = __shfl_sync(0xffffffffu, fmaf(-fb, ex, fmaf(-fa, dx, fjx)), src, kIL);
+    fjy = __shfl_sync(0xffffffffu, fmaf(-fb, ey, fmaf(-fa, dy, fjy)), src, kIL);
+    fjz = __shfl_sync(0xffffffffu, fmaf(-fb, ez, fmaf(-fa, dz, fjz)), src, kIL);
+  }
+}
+
+// bits of segment seg of an exclusion word, rotated so that bit k belongs to step k
+__device__ __forceinline__ uint32_t seg_mask(uint32_t excl, int seg, int il) {
+  constexpr uint32_t m = (1u << kIL) - 1u;
+  const uint32_t w = (excl >> (seg * kIL)) & m;
+  return ((w >> il) | (w << (kIL - il))) & m;
+}
+
+template <bool ENERGY>
+__device__ __forceinline__ void run_tile(const PairConst& c, const SysParams& p, const float4& x0, const float4& x1,
+                                         float q0, float q1, const char* lj0, const char* lj1, uint32_t je,
+                                         uint32_t ex0, uint32_t ex1, float4 xj, int tyj, float4* jx, int* jt,
+                                         const int* __restrict__ perm, long long* __restrict__ facc, int lane, int src,
+                                         float* f0, float* f1, float& ev, float& ee, float* vir) {
   const int jslot = (int)(je & kSlotMask);
   const int code = (int)(je >> kSlotBits);
   if (code != kNoShift) {
@@ -127,65 +185,21 @@ __device__ __forceinline__ void run_tile(const PairConst& c, const SysParams& p,
     xj.y += s.y;
     xj.z += s.z;
   }
-  const int il = lane & (kIG - 1), seg = (lane / kIG) * 2 * kIG;
+  const int il = lane & (kIL - 1), seg = lane / kIL;
+  float4* jxs = jx + seg * 2 * kIL + il;
+  int* jts = jt + seg * kTyStride + il;
   __syncwarp();
-  jx[seg + il] = xj;
-  jx[seg + il + kIG] = xj;
-  jt[seg + il] = tyj;
-  jt[seg + il + kIG] = tyj;
+  jxs[0] = xj;
+  jxs[kIL] = xj;
+  jts[0] = tyj * (int)sizeof(float2);
+  jts[kIL] = tyj * (int)sizeof(float2);
   __syncwarp();
-  // bit k of mrot: pair (il, entry h * kIG + (il + k) % kIG) excluded
-  uint32_t mrot;
-  if (kIG == 32) {
-    mrot = __funnelshift_r(excl, excl, il);
-  } else {
-    const uint32_t segm = (1u << (kIG & 31)) - 1u;
-    const uint32_t w = (excl >> ((lane / kIG) * kIG)) & segm;
-    mrot = ((w >> il) | (w << ((kIG - il) & 31))) & segm;
-  }
-  const float4* jxl = jx + seg + il;
-  const int* jtl = jt + seg + il;
+  const uint32_t m0 = seg_mask(ex0, seg, il), m1 = seg_mask(ex1, seg, il);
   float fjx = 0.f, fjy = 0.f, fjz = 0.f;
-  if (__any_sync(0xffffffffu, mrot != 0u)) {
-#pragma unroll 8
-    for (int k = 0; k < kIG; ++k) {
-      const float4 b = jxl[k];
-      const float dx = xi.x - b.x, dy = xi.y - b.y, dz = xi.z - b.z;
-      const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-      const bool ok = (r2 < c.rc2) && !((mrot >> k) & 1u);
-      const float fr = pair_force<ENERGY>(c, r2, qi * b.w, ljrow[jtl[k]], ok, ev, ee);
-      if (ENERGY) {
-        vir[0] = fmaf(fr * dx, dx, vir[0]);
-        vir[1] = fmaf(fr * dy, dy, vir[1]);
-        vir[2] = fmaf(fr * dz, dz, vir[2]);
-      }
-      fix = fmaf(fr, dx, fix);
-      fiy = fmaf(fr, dy, fiy);
-      fiz = fmaf(fr, dz, fiz);
-      fjx = __shfl_sync(0xffffffffu, fmaf(-fr, dx, fjx), src, kIG);
-      fjy = __shfl_sync(0xffffffffu, fmaf(-fr, dy, fjy), src, kIG);
-      fjz = __shfl_sync(0xffffffffu, fmaf(-fr, dz, fjz), src, kIG);
-    }
-  } else {
-#pragma unroll 8
-    for (int k = 0; k < kIG; ++k) {
-      const float4 b = jxl[k];
-      const float dx = xi.x - b.x, dy = xi.y - b.y, dz = xi.z - b.z;
-      const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-      const float fr = pair_force<ENERGY>(c, r2, qi * b.w, ljrow[jtl[k]], r2 < c.rc2, ev, ee);
-      if (ENERGY) {
-        vir[0] = fmaf(fr * dx, dx, vir[0]);
-        vir[1] = fmaf(fr * dy, dy, vir[1]);
-        vir[2] = fmaf(fr * dz, dz, vir[2]);
-      }
-      fix = fmaf(fr, dx, fix);
-      fiy = fmaf(fr, dy, fiy);
-      fiz = fmaf(fr, dz, fiz);
-      fjx = __shfl_sync(0xffffffffu, fmaf(-fr, dx, fjx), src, kIG);
-      fjy = __shfl_sync(0xffffffffu, fmaf(-fr, dy, fjy), src, kIG);
-      fjz = __shfl_sync(0xffffffffu, fmaf(-fr, dz, fjz), src, kIG);
-    }
-  }
+  if (__any_sync(0xffffffffu, (m0 | m1) != 0u))
+    tile_steps<ENERGY, true>(c, x0, x1, q0, q1, lj0, lj1, m0, m1, jxs, jts, src, f0, f1, ev, ee, vir, fjx, fjy, fjz);
+  else
+    tile_steps<ENERGY, false>(c, x0, x1, q0, q1, lj0, lj1, 0u, 0u, jxs, jts, src, f0, f1, ev, ee, vir, fjx, fjy, fjz);
   const int aj = perm[jslot];
   if (aj >= 0) {
     const int n = p.n;
@@ -207,7 +221,7 @@ __device__ __forceinline__ void nonbonded_body(const SysParams& p, const PairCon
   if (closing && threadIdx.x == 0) lists_close(closing, closing_prune, counters);
   extern __shared__ float2 lj[];
   __shared__ float4 jx_all[kWarps][64];
-  __shared__ int jt_all[kWarps][64];
+  __shared__ int jt_all[kWarps][kSeg * kTyStride];
   const int nt1 = p.ntypes + 1;
   for (int k = threadIdx.x; k < nt1 * nt1; k += blockDim.x) lj[k] = make_float2(6.f * ljtab[k].x, ljtab[k].y);
   __syncthreads();
@@ -216,8 +230,8 @@ __device__ __forceinline__ void nonbonded_body(const SysParams& p, const PairCon
   float4* jx = jx_all[warp];
   int* jt = jt_all[warp];
   const int n = p.n;
-  const int il = lane & (kIG - 1);
-  const int src = (il + 1) & (kIG - 1);  // segment-relative source lane of the j-force rotation
+  const int il = lane & (kIL - 1);
+  const int src = (il + 1) & (kIL - 1);  // segment-relative source lane of the j-force rotation
   // energy and virial sums per lane in fixed point, item by item: integer sums do not
   // depend on which items a warp happens to fetch, so energies are bit-reproducible
   long long e_vdw = 0, e_el = 0, w_acc[3] = {0, 0, 0};
@@ -229,12 +243,13 @@ __device__ __forceinline__ void nonbonded_body(const SysParams& p, const PairCon
     const int2 item = items[it];
     const int g = item.x;  // i-group: block I, atoms s * kIG .. s * kIG + kIG - 1
     const int I = g / kNG, s = g % kNG;
-    const int ib = s * kIG + il;  // this lane's i atom, index within the block
+    const int ib = s * kIG + il;  // this lane's first i atom, index within the block; the second is ib + kIL
     const int islot = I * 32 + ib;
-    const float4 xi = xyzq[islot];
-    const float2* ljrow = lj + typ[islot] * nt1;
-    const float qi = xi.w * p.cc;
-    float fix = 0.f, fiy = 0.f, fiz = 0.f;
+    const float4 x0 = xyzq[islot], x1 = xyzq[islot + kIL];
+    const char* lj0 = reinterpret_cast<const char*>(lj + typ[islot] * nt1);
+    const char* lj1 = reinterpret_cast<const char*>(lj + typ[islot + kIL] * nt1);
+    const float q0 = x0.w * p.cc, q1 = x1.w * p.cc;
+    float f0[3] = {0.f, 0.f, 0.f}, f1[3] = {0.f, 0.f, 0.f};
     float ev = 0.f, ee = 0.f, vir[3] = {0.f, 0.f, 0.f};
     // tile 0 of a group is the group against its own block (upper triangle j > i);
     // each tile's entry, exclusion word and j data are loaded one tile ahead
@@ -242,42 +257,47 @@ __device__ __forceinline__ void nonbonded_body(const SysParams& p, const PairCon
     const int tend = min(inner_nt[g] + 1, t + chunk);
     const uint32_t* jl = inner + (size_t)g * ocap - 32;  // inner tile t-1
     const int* ml = inner_m + (size_t)g * (ocap >> 5) - 1;
-    auto fetch = [&](int tt, uint32_t& je, uint32_t& ex, float4& xj, int& tyj) {
+    auto fetch = [&](int tt, uint32_t& je, uint32_t& ex0, uint32_t& ex1, float4& xj, int& tyj) {
       if (tt == 0) {
         je = (uint32_t)(I * 32 + lane) | ((uint32_t)kNoShift << kSlotBits);
-        ex = dmask[islot] | ((ib == 31) ? 0xffffffffu : ((2u << ib) - 1u));
+        ex0 = dmask[islot] | ((2u << ib) - 1u);
+        ex1 = dmask[islot + kIL] | ((ib + kIL == 31) ? 0xffffffffu : ((2u << (ib + kIL)) - 1u));
       } else {
         je = jl[tt * 32 + lane];
         const int m = ml[tt];
-        ex = m >= 0 ? masks[(size_t)m * kIG + il] : 0u;
+        ex0 = m >= 0 ? masks[(size_t)m * kIG + il] : 0u;
+        ex1 = m >= 0 ? masks[(size_t)m * kIG + il + kIL] : 0u;
       }
       xj = xyzq[je & kSlotMask];
       tyj = typ[je & kSlotMask];
     };
-    uint32_t je_n, ex_n;
+    uint32_t je_n, e0_n, e1_n;
     float4 xj_n;
     int ty_n;
-    fetch(t, je_n, ex_n, xj_n, ty_n);
+    fetch(t, je_n, e0_n, e1_n, xj_n, ty_n);
     for (; t < tend; ++t) {
-      const uint32_t je = je_n, ex = ex_n;
+      const uint32_t je = je_n, e0 = e0_n, e1 = e1_n;
       const float4 xj = xj_n;
       const int ty = ty_n;
-      if (t + 1 < tend) fetch(t + 1, je_n, ex_n, xj_n, ty_n);
-      run_tile<ENERGY>(c, p, xi, qi, ljrow, je, ex, xj, ty, jx, jt, perm, facc, lane, src, fix, fiy, fiz, ev, ee,
-                       vir);
+      if (t + 1 < tend) fetch(t + 1, je_n, e0_n, e1_n, xj_n, ty_n);
+      run_tile<ENERGY>(c, p, x0, x1, q0, q1, lj0, lj1, je, e0, e1, xj, ty, jx, jt, perm, facc, lane, src, f0, f1, ev,
+                       ee, vir);
     }
-    // the i force of lane il is split over the 32 / kIG segments
+    // the i forces are split over the segments; then lane l < kIG flushes i atom l
 #pragma unroll
-    for (int off = kIG; off < 32; off <<= 1) {
-      fix += __shfl_xor_sync(0xffffffffu, fix, off);
-      fiy += __shfl_xor_sync(0xffffffffu, fiy, off);
-      fiz += __shfl_xor_sync(0xffffffffu, fiz, off);
+    for (int d = 0; d < 3; ++d) {
+#pragma unroll
+      for (int off = kIL; off < 32; off <<= 1) {
+        f0[d] += __shfl_xor_sync(0xffffffffu, f0[d], off);
+        f1[d] += __shfl_xor_sync(0xffffffffu, f1[d], off);
+      }
     }
-    const int ai = perm[islot];
-    if (lane < kIG && ai >= 0) {
-      red_add(facc + ai, to_fix(fix));
-      red_add(facc + n + ai, to_fix(fiy));
-      red_add(facc + 2 * n + ai, to_fix(fiz));
+    const bool second = lane >= kIL;
+    const int ai = lane < kIG ? perm[I * 32 + s * kIG + lane] : -1;
+    if (ai >= 0) {
+      red_add(facc + ai, to_fix(second ? f1[0] : f0[0]));
+      red_add(facc + n + ai, to_fix(second ? f1[1] : f0[1]));
+      red_add(facc + 2 * n + ai, to_fix(second ? f1[2] : f0[2]));
     }
     if (ENERGY) {
       e_vdw += __double2ll_rn((double)ev * kFixE);
