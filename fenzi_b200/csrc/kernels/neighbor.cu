@@ -649,18 +649,21 @@ __device__ __forceinline__ void prune_body(const RebuildArgs& A, int bid, int nb
     ++ntile[s];
     __syncwarp();
   };
-  // the next chunk's entries and positions are loaded before this chunk's distance
-  // tests, so the gathers overlap the arithmetic
+  // the next chunk's positions are loaded before this chunk's distance tests, through
+  // entries loaded one chunk before that: a gather that waits for its own entries
+  // stalls the warp for an L2 round trip in every chunk
   const float rp2_keep = rp2 + 1e-3f;
   uint32_t e_nx = lane < n ? src[lane] : dummy;
+  uint32_t e_n2 = 32 + lane < n ? src[32 + lane] : dummy;
   float4 r_nx = xyzq_s[e_nx & kSlotMask];
   for (int c0 = 0; c0 < n; c0 += 32) {
     const bool valid = c0 + lane < n;
     const uint32_t e = e_nx;
     float4 r = r_nx;
     if (c0 + 32 < n) {
-      e_nx = c0 + 32 + lane < n ? src[c0 + 32 + lane] : dummy;
+      e_nx = e_n2;
       r_nx = xyzq_s[e_nx & kSlotMask];
+      e_n2 = c0 + 64 + lane < n ? src[c0 + 64 + lane] : dummy;
     }
     const int code = (int)(e >> kSlotBits);
     if (code != kNoShift) {
@@ -777,11 +780,17 @@ __device__ __forceinline__ void prune_split_body(const RebuildArgs& A, int I) {
   int count[kNG];
 #pragma unroll
   for (int s = 0; s < kNG; ++s) count[s] = 0;
+  // positions one chunk ahead, entries two (as the warp-per-block prune)
+  auto entry = [&](int c) { return c < c_end && c * 32 + lane < n ? src[c * 32 + lane] : dummy; };
+  uint32_t e_nx = entry(c_begin), e_n2 = entry(c_begin + 1);
+  float4 r_nx = A.xyzq_s[e_nx & kSlotMask];
   for (int c = c_begin; c < c_end; ++c) {
-    const int e_i = c * 32 + lane;
-    const bool valid = e_i < n;
-    const uint32_t e = valid ? src[e_i] : dummy;
-    float4 r = A.xyzq_s[e & kSlotMask];
+    const bool valid = c * 32 + lane < n;
+    const uint32_t e = e_nx;
+    float4 r = r_nx;
+    e_nx = e_n2;
+    r_nx = A.xyzq_s[e_nx & kSlotMask];
+    e_n2 = entry(c + 2);
     const int code = (int)(e >> kSlotBits);
     if (code != kNoShift) {
       const float3 sh = shift_of(code, p);
@@ -866,7 +875,7 @@ __device__ __forceinline__ void prune_split_body(const RebuildArgs& A, int I) {
   }
 }
 
-__global__ void __launch_bounds__(kPruneWarps * 32) k_prune_split(RebuildArgs a) {
+__global__ void __launch_bounds__(kPruneWarps * 32, 2) k_prune_split(RebuildArgs a) {
   griddep_wait();
   prune_split_body(a, blockIdx.x);
 }

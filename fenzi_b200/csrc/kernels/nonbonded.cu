@@ -179,6 +179,7 @@ __device__ __forceinline__ void run_tile(const PairConst& c, const SysParams& p,
                                          float* f0, float* f1, float& ev, float& ee, float* vir) {
   const int jslot = (int)(je & kSlotMask);
   const int code = (int)(je >> kSlotBits);
+  const int aj = perm[jslot];  // needed at the tile's end: asked for now
   if (code != kNoShift) {
     const float3 s = shift_of(code, p);
     xj.x += s.x;
@@ -200,7 +201,6 @@ __device__ __forceinline__ void run_tile(const PairConst& c, const SysParams& p,
     tile_steps<ENERGY, true>(c, x0, x1, q0, q1, lj0, lj1, m0, m1, jxs, jts, src, f0, f1, ev, ee, vir, fjx, fjy, fjz);
   else
     tile_steps<ENERGY, false>(c, x0, x1, q0, q1, lj0, lj1, 0u, 0u, jxs, jts, src, f0, f1, ev, ee, vir, fjx, fjy, fjz);
-  const int aj = perm[jslot];
   if (aj >= 0) {
     const int n = p.n;
     red_add(facc + aj, to_fix(fjx));
@@ -216,7 +216,7 @@ __device__ __forceinline__ void nonbonded_body(const SysParams& p, const PairCon
     const int* __restrict__ perm, const uint32_t* __restrict__ inner, const int* __restrict__ inner_nt,
     const int* __restrict__ inner_m, const uint32_t* __restrict__ dmask, const uint32_t* __restrict__ masks,
     int* __restrict__ counters, const int2* __restrict__ items, int chunk, const float2* __restrict__ ljtab,
-    long long* __restrict__ facc, long long* __restrict__ energy, int ocap, int* closing, int* closing_prune) {
+    long long* __restrict__ facc, long long* __restrict__ energy, int ocap, int* closing, int* closing_prune, int bid, int nbid) {
   griddep_wait();
   if (closing && threadIdx.x == 0) lists_close(closing, closing_prune, counters);
   extern __shared__ float2 lj[];
@@ -235,35 +235,42 @@ __device__ __forceinline__ void nonbonded_body(const SysParams& p, const PairCon
   // energy and virial sums per lane in fixed point, item by item: integer sums do not
   // depend on which items a warp happens to fetch, so energies are bit-reproducible
   long long e_vdw = 0, e_el = 0, w_acc[3] = {0, 0, 0};
-  for (;;) {
-    int it = 0;
-    if (lane == 0) it = atomicAdd(&counters[CNT_WORK], 1);
-    it = __shfl_sync(0xffffffffu, it, 0);
-    if (it >= nitems) break;
-    const int2 item = items[it];
-    const int g = item.x;  // i-group: block I, atoms s * kIG .. s * kIG + kIG - 1
+  // Work items: a warp starts with the item of its own number and takes further ones
+  // from the counter, each asked for while the last tile of the one before is worked on
+  // (asked for earlier, a warp holds an item that another could start on).  All warps
+  // starting at the counter queue at one L2 address: 3,500 warps for the few hundred
+  // items of a 648-atom system.
+  const int nwarps = nbid * kWarps;
+  int it = bid * kWarps + warp;
+  int2 item = it < nitems ? items[it] : make_int2(0, 0);
+  while (it < nitems) {
+    int it_next = nitems;
+    const int g = item.x, t_first = item.y;  // i-group: block I, atoms s * kIG .. s * kIG + kIG - 1
     const int I = g / kNG, s = g % kNG;
     const int ib = s * kIG + il;  // this lane's first i atom, index within the block; the second is ib + kIL
     const int islot = I * 32 + ib;
     const float4 x0 = xyzq[islot], x1 = xyzq[islot + kIL];
     const char* lj0 = reinterpret_cast<const char*>(lj + typ[islot] * nt1);
     const char* lj1 = reinterpret_cast<const char*>(lj + typ[islot + kIL] * nt1);
+    const int ai = lane < kIG ? perm[I * 32 + s * kIG + lane] : -1;
     const float q0 = x0.w * p.cc, q1 = x1.w * p.cc;
     float f0[3] = {0.f, 0.f, 0.f}, f1[3] = {0.f, 0.f, 0.f};
     float ev = 0.f, ee = 0.f, vir[3] = {0.f, 0.f, 0.f};
     // tile 0 of a group is the group against its own block (upper triangle j > i);
     // each tile's entry, exclusion word and j data are loaded one tile ahead
-    int t = item.y;
+    int t = t_first;
     const int tend = min(inner_nt[g] + 1, t + chunk);
     const uint32_t* jl = inner + (size_t)g * ocap - 32;  // inner tile t-1
     const int* ml = inner_m + (size_t)g * (ocap >> 5) - 1;
-    auto fetch = [&](int tt, uint32_t& je, uint32_t& ex0, uint32_t& ex1, float4& xj, int& tyj) {
+    // (and the entry of the tile after that, so that no load waits for its own address)
+    auto entry = [&](int tt) {
+      return tt == 0 ? (uint32_t)(I * 32 + lane) | ((uint32_t)kNoShift << kSlotBits) : jl[tt * 32 + lane];
+    };
+    auto fetch = [&](int tt, uint32_t je, uint32_t& ex0, uint32_t& ex1, float4& xj, int& tyj) {
       if (tt == 0) {
-        je = (uint32_t)(I * 32 + lane) | ((uint32_t)kNoShift << kSlotBits);
         ex0 = dmask[islot] | ((2u << ib) - 1u);
         ex1 = dmask[islot + kIL] | ((ib + kIL == 31) ? 0xffffffffu : ((2u << (ib + kIL)) - 1u));
       } else {
-        je = jl[tt * 32 + lane];
         const int m = ml[tt];
         ex0 = m >= 0 ? masks[(size_t)m * kIG + il] : 0u;
         ex1 = m >= 0 ? masks[(size_t)m * kIG + il + kIL] : 0u;
@@ -271,7 +278,7 @@ __device__ __forceinline__ void nonbonded_body(const SysParams& p, const PairCon
       xj = xyzq[je & kSlotMask];
       tyj = typ[je & kSlotMask];
     };
-    uint32_t je_n, e0_n, e1_n;
+    uint32_t je_n = entry(t), je_n2 = t + 1 < tend ? entry(t + 1) : 0u, e0_n, e1_n;
     float4 xj_n;
     int ty_n;
     fetch(t, je_n, e0_n, e1_n, xj_n, ty_n);
@@ -279,10 +286,18 @@ __device__ __forceinline__ void nonbonded_body(const SysParams& p, const PairCon
       const uint32_t je = je_n, e0 = e0_n, e1 = e1_n;
       const float4 xj = xj_n;
       const int ty = ty_n;
-      if (t + 1 < tend) fetch(t + 1, je_n, e0_n, e1_n, xj_n, ty_n);
+      if (t + 1 < tend) {
+        je_n = je_n2;
+        fetch(t + 1, je_n, e0_n, e1_n, xj_n, ty_n);
+        if (t + 2 < tend) je_n2 = entry(t + 2);
+      } else if (nitems > nwarps && lane == 0) {
+        it_next = nwarps + atomicAdd(&counters[CNT_WORK], 1);
+      }
       run_tile<ENERGY>(c, p, x0, x1, q0, q1, lj0, lj1, je, e0, e1, xj, ty, jx, jt, perm, facc, lane, src, f0, f1, ev,
                        ee, vir);
     }
+    it = __shfl_sync(0xffffffffu, it_next, 0);
+    if (it < nitems) item = items[it];
     // the i forces are split over the segments; then lane l < kIG flushes i atom l
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -293,7 +308,6 @@ __device__ __forceinline__ void nonbonded_body(const SysParams& p, const PairCon
       }
     }
     const bool second = lane >= kIL;
-    const int ai = lane < kIG ? perm[I * 32 + s * kIG + lane] : -1;
     if (ai >= 0) {
       red_add(facc + ai, to_fix(second ? f1[0] : f0[0]));
       red_add(facc + n + ai, to_fix(second ? f1[1] : f0[1]));
@@ -323,7 +337,7 @@ __global__ void __launch_bounds__(256, MINB)
                 int chunk, const float2* __restrict__ ljtab, long long* __restrict__ facc,
                 long long* __restrict__ energy, int ocap, int* flag, int* flag_prune) { griddep_wait();
   nonbonded_body<ENERGY>(p, c, xyzq, typ, perm, inner, inner_nt, inner_m, dmask, masks, counters, items, chunk, ljtab,
-                         facc, energy, ocap, blockIdx.x == 0 ? flag : nullptr, flag_prune);
+                         facc, energy, ocap, blockIdx.x == 0 ? flag : nullptr, flag_prune, blockIdx.x, gridDim.x);
 }
 
 // batched: every CTA serves one system's work queue (force variant only)
@@ -334,7 +348,7 @@ __global__ void __launch_bounds__(256, kNbBatchCtasPerSm) k_nonbonded_b(const No
   const PairConst c = pair_const(a.p);
   nonbonded_body<false>(a.p, c, a.xyzq_s, a.typ_s, a.perm, a.inner, a.inner_nt, a.inner_m, a.dmask, a.masks,
                         a.counters, a.items, a.chunk, a.ljtab, a.facc, a.energy, a.ocap,
-                        t.y == 0 ? a.flag : nullptr, a.flag_prune);
+                        t.y == 0 ? a.flag : nullptr, a.flag_prune, t.y, t.z);
 }
 
 void launch_nonbonded(const NonbondedArgs& a, bool energy, cudaStream_t st, bool zero_work) {
