@@ -59,6 +59,7 @@ struct BatchKernels {
   std::vector<fzk::ClassBatch> classes;
   std::vector<fzk::PmeSizeBatch> sizes;
   size_t spread_smem = 0;
+  int box_n = 0;  // largest grid of the members whose PME one block does
   int max_ntypes = 0;
   long long launches = 0;  // kernels one batched step launches
   // appends v to the image (256-byte aligned); *out is set once the arena is known
@@ -186,6 +187,12 @@ static bool batched_kernels_ok(const fz_batch* b) {
   return true;
 }
 
+// Members from which the PME of small grids is a block per member.  us a step, blocks /
+// launches: 6 boxes of 216 to 2,000 waters 137 / 137, 12: 175 / 194, 24: 236 / 255, 48: 342
+// / 365, 96: 583 / 632; 24 of 1,500 to 2,000: 293 / 307; 64 of 216 to 500: 225 / 240.  The
+// numbers are the same either way.
+constexpr int kBoxMembers = 8;
+
 static void add_blocks(std::vector<int4>& tab, int arg, int nblocks) {
   for (int k = 0; k < nblocks; ++k) tab.push_back(make_int4(arg, k, nblocks, 0));
 }
@@ -215,6 +222,10 @@ static fz_status build_batch_kernels(fz_batch* b) {
   // finished CTA's slot takes the next CTA of the launch, so members whose rounded
   // share of CTAs is short finish with the rest (one wave ends with the member of the
   // largest work per CTA, up to 1.5x the mean)
+  int box_members = kBoxMembers;
+  if (const char* v = std::getenv("FZ_BATCH_BOX")) box_members = std::max(1, std::atoi(v));
+  const bool use_box = ns >= box_members;
+  std::vector<std::pair<int, int>> boxes;  // (grid size, member)
   int nb_waves = 2;
   if (const char* v = std::getenv("FZ_BATCH_NB_WAVES")) nb_waves = std::max(1, std::min(16, std::atoi(v)));
   for (int i = 0; i < ns; ++i) {
@@ -244,7 +255,8 @@ static fz_status build_batch_kernels(fz_batch* b) {
     const fzk::PmeArgs& pa = pme.back();
     const int nbr = pa.nb[0] * pa.nb[1] * pa.nb[2];
     const long long kt = (long long)pa.K[0] * pa.K[1] * pa.K[2];
-    add_blocks(tabs[fzk::BT_ONE], i, 1);
+    const bool box = use_box && fzk::pme_box_ok(pa);
+    if (box) boxes.push_back({pa.K[0], i});
     add_blocks(tabs[fzk::BT_ATOMS256], i, (p.n + 255) / 256);
     add_blocks(tabs[fzk::BT_COLUMNS], i, p.ncol[0] * p.ncol[1]);
     add_blocks(tabs[fzk::BT_SLOTS256], i, (p.nslots + 255) / 256);
@@ -253,10 +265,14 @@ static fz_status build_batch_kernels(fz_batch* b) {
                std::max(1, (int)std::lround((double)e->n_sm * fzk::kNbBatchCtasPerSm * nb_waves * p.n /
                                             (double)std::max(1LL, natoms))));
     add_blocks(tabs[fzk::BT_BONDED], i, fzk::bonded_blocks(bd.back()));
-    add_blocks(tabs[fzk::BT_BRICKS256], i, (nbr + 255) / 256);
-    add_blocks(tabs[fzk::BT_BRICKS], i, nbr);
-    add_blocks(tabs[fzk::BT_GRID256], i, (int)std::min<long long>(64, (kt + 255) / 256));
-    bk->spread_smem = std::max(bk->spread_smem, fzk::pme_spread_smem(pa));
+    if (!box) {
+      add_blocks(tabs[fzk::BT_ONE], i, 1);
+      add_blocks(tabs[fzk::BT_PME_ATOMS256], i, (p.n + 255) / 256);
+      add_blocks(tabs[fzk::BT_BRICKS256], i, (nbr + 255) / 256);
+      add_blocks(tabs[fzk::BT_BRICKS], i, nbr);
+      add_blocks(tabs[fzk::BT_GRID256], i, (int)std::min<long long>(64, (kt + 255) / 256));
+      bk->spread_smem = std::max(bk->spread_smem, fzk::pme_spread_smem(pa));
+    }
     bk->max_ntypes = std::max(bk->max_ntypes, p.ntypes);
     const fzk::IntegrateArgs ia = e->int_args();
     for (int c = 0; c < ia.ncls; ++c) {
@@ -274,6 +290,7 @@ static fz_status build_batch_kernels(fz_batch* b) {
       add_blocks(acc->tab, (int)acc->args.size(), (x.u_end - x.u_begin + 127) / 128);
       acc->args.push_back(x);
     }
+    if (box) continue;
     SizeAcc* sa = nullptr;
     for (auto& q : sizes)
       if (q.N == pa.K[0]) sa = &q;
@@ -284,6 +301,9 @@ static fz_status build_batch_kernels(fz_batch* b) {
     add_blocks(sa->plane, i, pa.K[2]);
     add_blocks(sa->z, i, fzk::pme_z_groups(pa));
   }
+  std::sort(boxes.begin(), boxes.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
+  for (const auto& q : boxes) add_blocks(tabs[fzk::BT_BOX], q.second, 1);
+  bk->box_n = boxes.empty() ? 0 : boxes[0].first;
   fz_status r;
   if ((r = bk->upload(rb, &bk->rb)) || (r = bk->upload(nb, &bk->nb)) || (r = bk->upload(bd, &bk->bd)) ||
       (r = bk->upload(pme, &bk->pme)))
@@ -317,7 +337,8 @@ static fz_status build_batch_kernels(fz_batch* b) {
   }
   if ((r = bk->place(b->arena, b->master))) return r;
   bk->launches = 2 * (long long)bk->classes.size() + fzk::kRebuildLaunches +
-                 1 + (bk->t.n[fzk::BT_BONDED] > 0 ? 1 : 0) + 7 + 3 * (long long)bk->sizes.size();
+                 1 + (bk->t.n[fzk::BT_BONDED] > 0 ? 1 : 0) + (bk->t.n[fzk::BT_BOX] > 0 ? 1 : 0) +
+                 (bk->sizes.empty() ? 0 : 7 + 3 * (long long)bk->sizes.size());
   b->bk = std::move(bk);
   return FZ_OK;
 }
@@ -334,7 +355,7 @@ static void batched_step_body(fz_batch* b, cudaStream_t st, bool open = true, bo
   }
   cudaEventRecord(b->ev_fork, st);
   cudaStreamWaitEvent(b->aux, b->ev_fork, 0);
-  fzk::launch_pme_b(k.pme, k.t, k.sizes.data(), (int)k.sizes.size(), k.spread_smem, b->aux);
+  fzk::launch_pme_b(k.pme, k.t, k.sizes.data(), (int)k.sizes.size(), k.spread_smem, k.box_n, b->aux);
   fzk::launch_rebuild_b(k.rb, k.t, st);
   fzk::launch_nonbonded_b(k.nb, k.t, k.max_ntypes, st);
   fzk::launch_bonded_b(k.bd, k.t, st);

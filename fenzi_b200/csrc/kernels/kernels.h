@@ -16,7 +16,9 @@ constexpr int kRebuildLaunches = 6;  // launch_rebuild without its close, launch
 // in that system's own grid, that grid's size, 0).  Tables are built on the host from
 // the systems' sizes, one per per-system grid shape.
 enum : int {
-  BT_ONE = 0,     // one block per system
+  BT_ONE = 0,     // one block per system whose PME has brick lists
+  BT_PME_ATOMS256,  // (n + 255) / 256 of those systems
+  BT_BOX,         // one block per system whose PME is done by one block
   BT_ATOMS256,    // (n + 255) / 256
   BT_COLUMNS,     // x-y columns of the neighbour sort
   BT_SLOTS256,    // (sorted slots + 255) / 256
@@ -125,7 +127,8 @@ struct PmeArgs {
   long long* facc;
   long long* energy;
   int* status;
-  int gather;  // gather kernel: 1 one CTA per brick, 2 one thread per atom, 0 by atoms per brick
+  int gather;  // gather kernel: 1 one CTA per brick, 2 one thread per atom, 0 by atoms per brick,
+               // 3 as 2 without brick lists
 };
 // cleared: launch_pme_clear has already been queued for this evaluation
 void launch_pme(const PmeArgs& a, bool energy, cudaStream_t st, bool cleared = false);
@@ -153,7 +156,9 @@ bool pme_batchable(const PmeArgs& a);
 size_t pme_spread_smem(const PmeArgs& a);
 int pme_z_groups(const PmeArgs& a);
 void launch_pme_b(const PmeArgs* args, const BatchTables& t, const PmeSizeBatch* sizes, int nsizes,
-                  size_t spread_smem, cudaStream_t st);
+                  size_t spread_smem, int box_n, cudaStream_t st);
+// whether one block can do the whole sum in shared memory (small cubic grids)
+bool pme_box_ok(const PmeArgs& a);
 int pme_launches(const PmeArgs& a);
 
 struct BondedArgs {

@@ -24,17 +24,18 @@ struct FftPlan {
   int rad[12];
 };
 
+// (products and sums that several kernels must round alike are written as explicit FMAs:
+// left to the compiler, each kernel's contraction is its own)
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+  return make_float2(fmaf(a.x, b.x, -__fmul_rn(a.y, b.y)), fmaf(a.x, b.y, __fmul_rn(a.y, b.x)));
 }
 
 // base grid point k0 and fraction t of coordinate x along a dimension of K points
 __device__ __forceinline__ int grid_base(float x, float invL, int K, float* t) {
   float s = x * invL;
   s -= floorf(s);
-  const float u = s * (float)K;
-  int k0 = (int)u;
-  float f = u - (float)k0;
+  int k0 = (int)__fmul_rn(s, (float)K);
+  float f = fmaf(s, (float)K, -(float)k0);
   if (k0 >= K) {
     k0 -= K;
     f = 0.f;
@@ -769,16 +770,16 @@ __device__ __forceinline__ void small_dft(float2* v) {
     // sg * i * b1 = (-sg b1.y, sg b1.x)
     v[0] = make_float2(a0.x + b0.x, a0.y + b0.y);
     v[2] = make_float2(a0.x - b0.x, a0.y - b0.y);
-    v[1] = make_float2(a1.x - sg * b1.y, a1.y + sg * b1.x);
-    v[3] = make_float2(a1.x + sg * b1.y, a1.y - sg * b1.x);
+    v[1] = make_float2(fmaf(-sg, b1.y, a1.x), fmaf(sg, b1.x, a1.y));
+    v[3] = make_float2(fmaf(sg, b1.y, a1.x), fmaf(-sg, b1.x, a1.y));
   } else if constexpr (R == 3) {
     const float c1 = -0.5f, s1 = sg * 0.86602540378443865f;  // e^{sg 2 pi i/3}
     const float2 t = make_float2(v[1].x + v[2].x, v[1].y + v[2].y);
     const float2 d = make_float2(v[1].x - v[2].x, v[1].y - v[2].y);
-    const float2 m = make_float2(v[0].x + c1 * t.x, v[0].y + c1 * t.y);
+    const float2 m = make_float2(fmaf(c1, t.x, v[0].x), fmaf(c1, t.y, v[0].y));
     v[0] = make_float2(v[0].x + t.x, v[0].y + t.y);
-    v[1] = make_float2(m.x - s1 * d.y, m.y + s1 * d.x);
-    v[2] = make_float2(m.x + s1 * d.y, m.y - s1 * d.x);
+    v[1] = make_float2(fmaf(-s1, d.y, m.x), fmaf(s1, d.x, m.y));
+    v[2] = make_float2(fmaf(s1, d.y, m.x), fmaf(-s1, d.x, m.y));
   } else {  // R == 5
     const float c1 = 0.30901699437494742f, c2 = -0.80901699437494742f;
     const float s1 = sg * 0.95105651629515357f, s2 = sg * 0.58778525229247313f;
@@ -786,10 +787,10 @@ __device__ __forceinline__ void small_dft(float2* v) {
     const float2 d1 = make_float2(v[1].x - v[4].x, v[1].y - v[4].y);
     const float2 t2 = make_float2(v[2].x + v[3].x, v[2].y + v[3].y);
     const float2 d2 = make_float2(v[2].x - v[3].x, v[2].y - v[3].y);
-    const float2 m1 = make_float2(v[0].x + c1 * t1.x + c2 * t2.x, v[0].y + c1 * t1.y + c2 * t2.y);
-    const float2 m2 = make_float2(v[0].x + c2 * t1.x + c1 * t2.x, v[0].y + c2 * t1.y + c1 * t2.y);
-    const float2 n1 = make_float2(s1 * d1.x + s2 * d2.x, s1 * d1.y + s2 * d2.y);
-    const float2 n2 = make_float2(s2 * d1.x - s1 * d2.x, s2 * d1.y - s1 * d2.y);
+    const float2 m1 = make_float2(fmaf(c2, t2.x, fmaf(c1, t1.x, v[0].x)), fmaf(c2, t2.y, fmaf(c1, t1.y, v[0].y)));
+    const float2 m2 = make_float2(fmaf(c1, t2.x, fmaf(c2, t1.x, v[0].x)), fmaf(c1, t2.y, fmaf(c2, t1.y, v[0].y)));
+    const float2 n1 = make_float2(fmaf(s1, d1.x, __fmul_rn(s2, d2.x)), fmaf(s1, d1.y, __fmul_rn(s2, d2.y)));
+    const float2 n2 = make_float2(fmaf(s2, d1.x, -__fmul_rn(s1, d2.x)), fmaf(s2, d1.y, -__fmul_rn(s1, d2.y)));
     v[0] = make_float2(v[0].x + t1.x + t2.x, v[0].y + t1.y + t2.y);
     v[1] = make_float2(m1.x - n1.y, m1.y + n1.x);
     v[4] = make_float2(m1.x + n1.y, m1.y - n1.x);
@@ -1166,6 +1167,266 @@ __global__ void __launch_bounds__(kPlaneThreads) k_fft_yx_plane_b(const PmeArgs*
   X(16) X(18) X(20) X(24) X(25) X(27) X(30) X(32) X(36) X(40) X(45) X(48) X(50) X(54) X(60) X(64) X(72) X(80) \
   X(90) X(96) X(100) X(108) X(120) X(128)
 
+// ------------------------------------------------------------------ a box in one block
+// The whole reciprocal sum of a batch member's small cubic grid by one block: the grid
+// lives in its shared memory from the spread to the gather.  Rows of N charges (int32, then float
+// potentials) and of N/2 + 1 complex numbers share their place, `pitch` float2 apart
+// (odd, to spread rows over the banks).  A thread takes a whole line through its DFT in
+// registers (the stages, radices and row pairing of the plane and z kernels, so the
+// potentials are the same numbers) and puts it back where it was; the z pass does both
+// directions with the influence function between them.
+// What it replaces: ten launches, then three for every grid size among the members, each
+// of them short of work (a 27^3 plane keeps 14 lines busy in a block of 1,024 threads) and
+// each a round trip of the grids through L2.  128 boxes of 216 to 2,000 waters: 806 -> 748
+// us a step; bound by its largest member (a block per SM).  One box alone is faster with
+// the launches (648 atoms: 26.3 against 29.4 us a step).
+constexpr int kBoxThreads = 640;  // 544 lines at N = 32; 96 registers a thread
+#define FZ_BOX_SIZES(X) X(16) X(18) X(20) X(24) X(25) X(27) X(30) X(32) X(36)
+
+__host__ __device__ constexpr int box_pitch(int n) { return (n / 2 + 1) | 1; }
+static size_t box_smem(int n) { return (size_t)n * n * box_pitch(n) * sizeof(float2) + n * sizeof(float2) + 6 * n * sizeof(float); }
+
+template <int N, int S, int NS, bool INV>
+__device__ __forceinline__ void fft_regs(float2* v, const float2* tw) {
+  if constexpr (S < nstages(N)) {
+    constexpr int R = radix_at(N, S), NB = N / R, STEP = N / (NS * R);
+    float2 w[N];
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+      const int k = j % NS;
+      float2 u[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        u[r] = v[j + r * NB];
+        if (r > 0 && k > 0) {
+          float2 t = tw[r * k * STEP];
+          if (INV) t.y = -t.y;
+          u[r] = cmul(u[r], t);
+        }
+      }
+      small_dft<R, INV>(u);
+      const int o = (j / NS) * NS * R + k;
+#pragma unroll
+      for (int r = 0; r < R; ++r) w[o + r * NS] = u[r];
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = w[i];
+    fft_regs<N, S + 1, NS * R, INV>(v, tw);
+  }
+}
+
+template <int N>
+__device__ __noinline__ void pme_box_body(const PmeArgs& a) {
+  extern __shared__ float2 sm[];
+  constexpr int NH = N / 2 + 1, P = box_pitch(N), NP = (N + 1) / 2, ROW = 2 * P;
+  float2* C = sm;                                    // [z][y][mx], rows P apart
+  float2* tw = sm + (size_t)N * N * P;
+  float* tab = reinterpret_cast<float*>(tw + N);     // gfac x, y, z, f2 x, y, z
+  int* Q = reinterpret_cast<int*>(sm);
+  const float* phi = reinterpret_cast<const float*>(sm);
+  const int tid = threadIdx.x;
+  for (int k = tid; k < N * N * ROW; k += kBoxThreads) Q[k] = 0;
+  for (int k = tid; k < N; k += kBoxThreads) {
+    tw[k] = a.tw[0][k];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      tab[d * N + k] = a.gfac[d][k];
+      tab[(3 + d) * N + k] = a.f2[d][k];
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < a.n; i += kBoxThreads) {
+    const float4 r = a.pos4[i];
+    float tx, ty, tz, wx[4], wy[4], wz[4];
+    const int kx = grid_base(r.x, a.p.inv_box.x, N, &tx);
+    const int ky = grid_base(r.y, a.p.inv_box.y, N, &ty);
+    const int kz = grid_base(r.z, a.p.inv_box.z, N, &tz);
+    bsp4(tx, wx, nullptr);
+    bsp4(ty, wy, nullptr);
+    bsp4(tz, wz, nullptr);
+    const float q = r.w * kFixQ32;
+#pragma unroll
+    for (int jz = 0; jz < 4; ++jz) {
+      int z = kz - jz;
+      z += z < 0 ? N : 0;
+#pragma unroll
+      for (int jy = 0; jy < 4; ++jy) {
+        int y = ky - jy;
+        y += y < 0 ? N : 0;
+        const float qzy = q * wz[jz] * wy[jy];
+        int* row = Q + (z * N + y) * ROW;
+#pragma unroll
+        for (int jx = 0; jx < 4; ++jx) {
+          int x = kx - jx;
+          x += x < 0 ? N : 0;
+          atomicAdd(row + x, __float2int_rn(qzy * wx[jx]));
+        }
+      }
+    }
+  }
+  __syncthreads();
+  // x forward, rows (2l, 2l + 1) of a plane per thread
+  for (int t = tid; t < N * NP; t += kBoxThreads) {
+    const int z = t / NP, l = t - z * NP;
+    const int r0 = (z * N + 2 * l) * ROW;
+    const bool two = 2 * l + 1 < N;
+    float2 v[N];
+#pragma unroll
+    for (int x = 0; x < N; ++x)
+      v[x] = make_float2((float)Q[r0 + x] * (1.0f / kFixQ32), two ? (float)Q[r0 + ROW + x] * (1.0f / kFixQ32) : 0.f);
+    fft_regs<N, 0, 1, false>(v, tw);
+    float2* o = C + (z * N + 2 * l) * P;
+#pragma unroll
+    for (int m = 0; m < NH; ++m) {
+      const float2 u = v[m], w = v[m == 0 ? 0 : N - m];
+      o[m] = make_float2(0.5f * (u.x + w.x), 0.5f * (u.y - w.y));
+      if (two) o[P + m] = make_float2(0.5f * (u.y + w.y), 0.5f * (w.x - u.x));
+    }
+  }
+  __syncthreads();
+  for (int t = tid; t < N * NH; t += kBoxThreads) {
+    const int z = t / NH, m = t - z * NH;
+    float2* o = C + z * N * P + m;
+    float2 v[N];
+#pragma unroll
+    for (int y = 0; y < N; ++y) v[y] = o[y * P];
+    fft_regs<N, 0, 1, false>(v, tw);
+#pragma unroll
+    for (int y = 0; y < N; ++y) o[y * P] = v[y];
+  }
+  __syncthreads();
+  for (int t = tid; t < N * NH; t += kBoxThreads) {
+    const int y = t / NH, mx = t - y * NH;
+    float2* o = C + y * P + mx;
+    float2 v[N];
+#pragma unroll
+    for (int z = 0; z < N; ++z) v[z] = o[z * N * P];
+    fft_regs<N, 0, 1, false>(v, tw);
+    const float gx = tab[mx], gy = tab[N + y], fx2 = tab[3 * N + mx], fy2 = tab[4 * N + y];
+#pragma unroll
+    for (int z = 0; z < N; ++z) {
+      float G = 0.f;
+      if ((mx | y | z) != 0) G = a.gscale * gx * gy * tab[2 * N + z] / (fx2 + fy2 + tab[5 * N + z]);
+      v[z].x = __fmul_rn(v[z].x, G);  // rounded before the next stage adds, as where it is stored
+      v[z].y = __fmul_rn(v[z].y, G);
+    }
+    fft_regs<N, 0, 1, true>(v, tw);
+#pragma unroll
+    for (int z = 0; z < N; ++z) o[z * N * P] = v[z];
+  }
+  __syncthreads();
+  for (int t = tid; t < N * NH; t += kBoxThreads) {
+    const int z = t / NH, m = t - z * NH;
+    float2* o = C + z * N * P + m;
+    float2 v[N];
+#pragma unroll
+    for (int y = 0; y < N; ++y) v[y] = o[y * P];
+    fft_regs<N, 0, 1, true>(v, tw);
+#pragma unroll
+    for (int y = 0; y < N; ++y) o[y * P] = v[y];
+  }
+  __syncthreads();
+  for (int t = tid; t < N * NP; t += kBoxThreads) {
+    const int z = t / NP, l = t - z * NP;
+    const float2* o = C + (z * N + 2 * l) * P;
+    const bool two = 2 * l + 1 < N;
+    float2 v[N];
+#pragma unroll
+    for (int m = 0; m < N; ++m) {
+      const bool lo = m < NH;
+      const int mm = lo ? m : N - m;
+      float2 x0 = o[mm], x1 = two ? o[P + mm] : make_float2(0.f, 0.f);
+      if (!lo) {
+        x0.y = -x0.y;
+        x1.y = -x1.y;
+      }
+      v[m] = make_float2(x0.x - x1.y, x0.y + x1.x);
+    }
+    fft_regs<N, 0, 1, true>(v, tw);
+    float* row = reinterpret_cast<float*>(sm) + (z * N + 2 * l) * ROW;
+#pragma unroll
+    for (int x = 0; x < N; ++x) {
+      row[x] = v[x].x;
+      if (two) row[ROW + x] = v[x].y;
+    }
+  }
+  __syncthreads();
+  const int n = a.n;
+  for (int i = tid; i < n; i += kBoxThreads) {
+    const float4 r = a.pos4[i];
+    float tx, ty, tz, wx[4], wy[4], wz[4], dx[4], dy[4], dz[4];
+    const int kx = grid_base(r.x, a.p.inv_box.x, N, &tx);
+    const int ky = grid_base(r.y, a.p.inv_box.y, N, &ty);
+    const int kz = grid_base(r.z, a.p.inv_box.z, N, &tz);
+    bsp4(tx, wx, dx);
+    bsp4(ty, wy, dy);
+    bsp4(tz, wz, dz);
+    // layer sums as (l0 + l1) + (l2 + l3), the order of every gather
+    float gx = 0.f, gy = 0.f, gz = 0.f, hx = 0.f, hy = 0.f, hz = 0.f;
+#pragma unroll
+    for (int jz = 0; jz < 4; ++jz) {
+      int z = kz - jz;
+      z += z < 0 ? N : 0;
+      float lx = 0.f, ly = 0.f, lz = 0.f;
+#pragma unroll
+      for (int jy = 0; jy < 4; ++jy) {
+        int y = ky - jy;
+        y += y < 0 ? N : 0;
+        const float* row = phi + (z * N + y) * ROW;
+        float sx = 0.f, sdx = 0.f;
+#pragma unroll
+        for (int jx = 0; jx < 4; ++jx) {
+          int x = kx - jx;
+          x += x < 0 ? N : 0;
+          const float f = row[x];
+          sx = fmaf(wx[jx], f, sx);
+          sdx = fmaf(dx[jx], f, sdx);
+        }
+        lx = fmaf(sdx, wy[jy] * wz[jz], lx);
+        ly = fmaf(sx, dy[jy] * wz[jz], ly);
+        lz = fmaf(sx, wy[jy] * dz[jz], lz);
+      }
+      if (jz == 0 || jz == 2) {
+        (jz == 0 ? gx : hx) = lx;
+        (jz == 0 ? gy : hy) = ly;
+        (jz == 0 ? gz : hz) = lz;
+      } else {
+        (jz == 1 ? gx : hx) += lx;
+        (jz == 1 ? gy : hy) += ly;
+        (jz == 1 ? gz : hz) += lz;
+      }
+    }
+    gx += hx;
+    gy += hy;
+    gz += hz;
+    const float q = r.w;
+    red_add(a.facc + i, to_fix(-q * gx * (float)N * a.p.inv_box.x));
+    red_add(a.facc + n + i, to_fix(-q * gy * (float)N * a.p.inv_box.y));
+    red_add(a.facc + 2 * n + i, to_fix(-q * gz * (float)N * a.p.inv_box.z));
+  }
+}
+
+// members of all sizes in one launch, a block each (the largest first)
+__global__ void __launch_bounds__(kBoxThreads) k_pme_box_b(const PmeArgs* __restrict__ args, const int4* __restrict__ tab) {
+  griddep_wait();
+  const PmeArgs& a = args[tab[blockIdx.x].x];
+  switch (a.K[0]) {
+#define FZ_C(N) case N: pme_box_body<N>(a); break;
+    FZ_BOX_SIZES(FZ_C)
+#undef FZ_C
+  }
+}
+
+bool pme_box_ok(const PmeArgs& a) {
+  if (a.K[0] != a.K[1] || a.K[0] != a.K[2]) return false;
+  switch (a.K[0]) {
+#define FZ_C(N) case N: return true;
+    FZ_BOX_SIZES(FZ_C)
+#undef FZ_C
+  }
+  return false;
+}
+
 static bool fft_x_r2c_t(const PmeArgs& a, int nl, dim3 g, size_t sm, cudaStream_t st) {
   switch (a.K[0]) {
 #define FZ_C(N) case N: launch_pdl(k_fft_x_r2c_t<N>, dim3(g), dim3(256), sm, st, a, nl); return true;
@@ -1371,11 +1632,17 @@ int pme_z_groups(const PmeArgs& a) {
 bool pme_batchable(const PmeArgs& a) { return use_plane_fft(a) && a.K[2] == a.K[0]; }
 
 void launch_pme_b(const PmeArgs* args, const BatchTables& t, const PmeSizeBatch* sizes, int nsizes,
-                  size_t spread_smem, cudaStream_t st) {
+                  size_t spread_smem, int box_n, cudaStream_t st) {
+  if (t.n[BT_BOX] > 0) {
+    const size_t sm = box_smem(box_n);
+    cudaFuncSetAttribute(k_pme_box_b, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)box_smem(36));
+    launch_pdl(k_pme_box_b, dim3(t.n[BT_BOX]), dim3(kBoxThreads), sm, st, args, t.tab[BT_BOX]);
+  }
+  if (t.n[BT_BRICKS] == 0) return;
   launch_pdl(k_pme_zero_b, dim3(t.n[BT_BRICKS256]), dim3(256), 0, st, args, t.tab[BT_BRICKS256]);
-  launch_pdl(k_pme_bin_b, dim3(t.n[BT_ATOMS256]), dim3(256), 0, st, args, t.tab[BT_ATOMS256]);
+  launch_pdl(k_pme_bin_b, dim3(t.n[BT_PME_ATOMS256]), dim3(256), 0, st, args, t.tab[BT_PME_ATOMS256]);
   launch_pdl(k_pme_scan_b, dim3(t.n[BT_ONE]), dim3(1024), 0, st, args, t.tab[BT_ONE]);
-  launch_pdl(k_pme_scatter_b, dim3(t.n[BT_ATOMS256]), dim3(256), 0, st, args, t.tab[BT_ATOMS256]);
+  launch_pdl(k_pme_scatter_b, dim3(t.n[BT_PME_ATOMS256]), dim3(256), 0, st, args, t.tab[BT_PME_ATOMS256]);
   launch_pdl(k_grid_zero_b, dim3(t.n[BT_GRID256]), dim3(256), 0, st, args, t.tab[BT_GRID256]);
   launch_pdl(k_pme_spread_b, dim3(t.n[BT_BRICKS]), dim3(256), spread_smem, st, args, t.tab[BT_BRICKS]);
   for (int pass = 0; pass < 3; ++pass)
