@@ -357,8 +357,47 @@ __device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefe
 // per term, 7 loads of atom pairs and 45 atomic adds per water in a launch of its own
 // (230,400 atoms: 17 us; 9,000 atoms: 6 us on the critical path); here the positions
 // are in registers and nothing is atomic.
-__device__ __forceinline__ void water_terms(const IntegrateArgs& a, int u, const Unit& U, const float4* x) {
+//
+// LPW lanes work on a water (1 or 4, neighbours in the warp, all with the same unit and
+// positions).  With 4, lane k < 3 takes pair k (bond and exclusion), lane 3 the angle,
+// and lane k stores atom k: a small system has too few waters to fill the GPU and its
+// pass lasts as long as one thread's chain of FP64 operations.
+__device__ __forceinline__ void pair_terms(const IntegrateArgs& a, const UnitTerms& T, const float4* x, const double* d,
+                                           int k, int i, int j, long long* g) {
+  g[0] = g[1] = g[2] = 0;
+  if (T.has >> k & 1) {
+    const float3 e = make_float3((float)d[0], (float)d[1], (float)d[2]);
+    float dr;
+    const float h = bond_force(e, T.bond[k], &dr);
+    g[0] += to_fix(h * e.x), g[1] += to_fix(h * e.y), g[2] += to_fix(h * e.z);
+  }
+  if (T.has >> (5 + k) & 1) {
+    const double r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+    double rr, erfv;
+    const double h = excl_force(r2, (double)x[i].w * (double)x[j].w, (double)a.p.beta, &rr, &erfv);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) g[c] += to_fix_d(h * d[c]);
+  }
+}
+
+// fixed-point angle forces on atoms 0, 1, 2 (d01, d02: atom 0 minus atoms 1, 2)
+__device__ __forceinline__ void apex_terms(const UnitTerms& T, const double* d01, const double* d02, long long f[3][3]) {
+  const bool swap = T.has >> 4 & 1;  // the angle's own order of its ends
+  const float3 e1 = make_float3(-(float)d01[0], -(float)d01[1], -(float)d01[2]);
+  const float3 e2 = make_float3(-(float)d02[0], -(float)d02[1], -(float)d02[2]);
+  float3 fi, fk;
+  float dth;
+  angle_force(swap ? e2 : e1, swap ? e1 : e2, T.angle, &fi, &fk, &dth);
+  const float3 f1 = swap ? fk : fi, f2 = swap ? fi : fk;
+  f[1][0] += to_fix(f1.x), f[1][1] += to_fix(f1.y), f[1][2] += to_fix(f1.z);
+  f[2][0] += to_fix(f2.x), f[2][1] += to_fix(f2.y), f[2][2] += to_fix(f2.z);
+  f[0][0] += to_fix(-fi.x - fk.x), f[0][1] += to_fix(-fi.y - fk.y), f[0][2] += to_fix(-fi.z - fk.z);
+}
+
+template <int LPW>
+__device__ __forceinline__ void water_terms(const IntegrateArgs& a, int u, const Unit& U, const float4* x, int q) {
   long long f[3][3] = {};
+  const int n = a.p.n;
   const int t = a.unit_term_of[u - a.unit_term_begin];
   if (t >= 0) {
     const UnitTerms T = a.unit_terms[t];
@@ -374,48 +413,53 @@ __device__ __forceinline__ void water_terms(const IntegrateArgs& a, int u, const
 #pragma unroll
       for (int c = 0; c < 3; ++c) d[k][c] -= L[c] * rint(d[k][c] * a.inv_box_d[c]);
     }
+    if constexpr (LPW == 1) {
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const int i = k == 2 ? 1 : 0, j = k == 0 ? 1 : 2;
-      const float3 e = make_float3((float)d[k][0], (float)d[k][1], (float)d[k][2]);
-      if (T.has >> k & 1) {
-        float dr;
-        const float g = bond_force(e, T.bond[k], &dr);
-        const long long g0 = to_fix(g * e.x), g1 = to_fix(g * e.y), g2 = to_fix(g * e.z);
-        f[i][0] += g0, f[i][1] += g1, f[i][2] += g2;
-        f[j][0] -= g0, f[j][1] -= g1, f[j][2] -= g2;
-      }
-      if (T.has >> (5 + k) & 1) {
-        const double r2 = d[k][0] * d[k][0] + d[k][1] * d[k][1] + d[k][2] * d[k][2];
-        double rr, erfv;
-        const double g = excl_force(r2, (double)x[i].w * (double)x[j].w, (double)p.beta, &rr, &erfv);
+      for (int k = 0; k < 3; ++k) {
+        const int i = k == 2 ? 1 : 0, j = k == 0 ? 1 : 2;
+        long long g[3];
+        pair_terms(a, T, x, d[k], k, i, j, g);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-          const long long gc = to_fix_d(g * d[k][c]);
-          f[i][c] += gc;
-          f[j][c] -= gc;
+          f[i][c] += g[c];
+          f[j][c] -= g[c];
         }
       }
-    }
-    if (T.has >> 3 & 1) {
-      const bool swap = T.has >> 4 & 1;
-      // base - apex; the angle's own order of its ends
-      const float3 e1 = make_float3(-(float)d[0][0], -(float)d[0][1], -(float)d[0][2]);
-      const float3 e2 = make_float3(-(float)d[1][0], -(float)d[1][1], -(float)d[1][2]);
-      float3 fi, fk;
-      float dth;
-      angle_force(swap ? e2 : e1, swap ? e1 : e2, T.angle, &fi, &fk, &dth);
-      const float3 f1 = swap ? fk : fi, f2 = swap ? fi : fk;
-      f[1][0] += to_fix(f1.x), f[1][1] += to_fix(f1.y), f[1][2] += to_fix(f1.z);
-      f[2][0] += to_fix(f2.x), f[2][1] += to_fix(f2.y), f[2][2] += to_fix(f2.z);
-      f[0][0] += to_fix(-fi.x - fk.x), f[0][1] += to_fix(-fi.y - fk.y), f[0][2] += to_fix(-fi.z - fk.z);
+      if (T.has >> 3 & 1) apex_terms(T, d[0], d[1], f);
+    } else {
+      const unsigned mask = 0xfu << (threadIdx.x & 28);
+      const int k = min(q, 2);
+      double dk[3];
+      float4 y[2];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) dk[c] = k == 0 ? d[0][c] : (k == 1 ? d[1][c] : d[2][c]);
+      y[0] = k == 2 ? x[1] : x[0];
+      y[1] = k == 0 ? x[1] : x[2];
+      UnitTerms Tk = T;
+      Tk.bond[0] = k == 0 ? T.bond[0] : (k == 1 ? T.bond[1] : T.bond[2]);
+      Tk.has = ((T.has >> k) & 1) | (((T.has >> (5 + k)) & 1) << 5);
+      long long g[3] = {0, 0, 0};
+      if (q < 3) pair_terms(a, Tk, y, dk, 0, 0, 1, g);
+      else if (T.has >> 3 & 1) apex_terms(T, d[0], d[1], f);
+      // atom 0: pairs 0 + 1, atom 1: pair 2 - pair 0, atom 2: - pair 1 - pair 2; and the angle
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const long long g0 = __shfl_sync(mask, g[c], 0, 4), g1 = __shfl_sync(mask, g[c], 1, 4),
+                        g2 = __shfl_sync(mask, g[c], 2, 4);
+        const long long a0 = __shfl_sync(mask, f[0][c], 3, 4), a1 = __shfl_sync(mask, f[1][c], 3, 4),
+                        a2 = __shfl_sync(mask, f[2][c], 3, 4);
+        f[0][c] = g0 + g1 + a0;
+        f[1][c] = g2 - g0 + a1;
+        f[2][c] = a2 - g1 - g2;
+      }
     }
   }
-  const int n = a.p.n;
 #pragma unroll
-  for (int k = 0; k < 3; ++k)
+  for (int k = 0; k < 3; ++k) {
+    if (LPW > 1 && q != k) continue;
 #pragma unroll
     for (int c = 0; c < 3; ++c) a.facc[(size_t)c * n + U.atom[k]] = f[k][c];
+  }
 }
 
 // NPT (Andersen barostat step with the integration units as scaling groups): the unit
@@ -425,11 +469,12 @@ __device__ __forceinline__ void water_terms(const IntegrateArgs& a, int u, const
 // pass does (half kick with the same forces, velocity constraints, velocities rounded
 // to the stored float), so one pass replaces the previous step's closing launch and
 // this step's opening one with bit-identical results.
-template <bool NPT, int NA, int NC, bool SETTLE, bool CLOSE = false>
+template <bool NPT, int NA, int NC, bool SETTLE, bool CLOSE = false, int LPW = 1>
 __device__ __forceinline__ void kick_drift_body(const IntegrateArgs& a, int u_begin, int u_end, int bid) {
   static_assert(!(NPT && CLOSE), "the closing pass is for constant-volume steps");
   griddep_wait();
-  const int u = u_begin + bid * blockDim.x + threadIdx.x;
+  // LPW lanes of a warp per unit, all doing the same up to the stores
+  const int u = u_begin + (bid * blockDim.x + threadIdx.x) / LPW, q_lane = threadIdx.x % LPW;
   if (u >= u_end) return;
   const Unit U = load_unit<NA, NC>(a, u);
   const int n = a.p.n;
@@ -459,6 +504,8 @@ __device__ __forceinline__ void kick_drift_body(const IntegrateArgs& a, int u_be
       r0[k][2] = pr.z;
     }
   }
+  // every lane of the unit has its loads before any of them stores
+  if (LPW > 1) __syncwarp(((1u << LPW) - 1u) << (threadIdx.x & 31 & ~(LPW - 1)));
   if (CLOSE) {
 #pragma unroll
     for (int k = 0; k < 4; ++k)
@@ -516,7 +563,7 @@ __device__ __forceinline__ void kick_drift_body(const IntegrateArgs& a, int u_be
     int st;
     if constexpr (SETTLE) st = settle_unit(U, r0, rn, im, a) ? 0 : 1;
     else st = shake_unit(U, r0, rn, im, a);
-    if (st) atomicOr(a.status, ST_SHAKE_NOCONV);
+    if (st && q_lane == 0) atomicOr(a.status, ST_SHAKE_NOCONV);
     const double idt = 1.0 / a.dtu;
 #pragma unroll
     for (int k = 0; k < 4; ++k)
@@ -531,6 +578,7 @@ __device__ __forceinline__ void kick_drift_body(const IntegrateArgs& a, int u_be
     const int i = U.atom[k];
     const float4 np = make_float4((float)rn[k][0], (float)rn[k][1], (float)rn[k][2], q[k]);
     x[k] = np;
+    if (LPW > 1 && q_lane != k) continue;
     a.pos4[i] = np;
     a.pos_drift[i] = np;
     a.vel4[i] = make_float4((float)v[k][0], (float)v[k][1], (float)v[k][2], (float)im[k]);
@@ -549,12 +597,19 @@ __device__ __forceinline__ void kick_drift_body(const IntegrateArgs& a, int u_be
   if (__any_sync(am, far) && lead) *a.flag = 1;
   if (__any_sync(am, moved) && lead) *a.flag_prune = 1;
   if constexpr (SETTLE) {
-    if (a.fuse_terms) water_terms(a, u, U, x);
+    if (a.fuse_terms) water_terms<LPW>(a, u, U, x, q_lane);
   }
 }
 
 template <bool NPT, int NA, int NC, bool SETTLE = false>
 __global__ void __launch_bounds__(128) k_kick_drift(IntegrateArgs a) { griddep_wait(); kick_drift_body<NPT, NA, NC, SETTLE>(a, a.u_begin, a.u_end, blockIdx.x); }
+
+// SETTLE waters alone (the one class of a water box), LPW lanes each
+template <bool NPT, bool CLOSE, int LPW>
+__global__ void __launch_bounds__(128, 4) k_drift_water(const __grid_constant__ IntegrateArgs a) {
+  griddep_wait();
+  kick_drift_body<NPT, 3, 3, true, CLOSE, LPW>(a, a.u_begin, a.u_end, blockIdx.x);
+}
 
 template <int NA, int NC, bool SETTLE>
 __global__ void __launch_bounds__(128, SETTLE ? 4 : 1) k_close_kick_drift(IntegrateArgs a) {
@@ -564,11 +619,11 @@ __global__ void __launch_bounds__(128, SETTLE ? 4 : 1) k_close_kick_drift(Integr
 
 // free atoms (class 0) and SETTLE waters (class 1), the two classes of a solvated system
 // without other hydrogens, in one launch: the waters' blocks first, then the free atoms'
-template <bool NPT, bool CLOSE>
+template <bool NPT, bool CLOSE, int LPW>
 __global__ void __launch_bounds__(128, 4) k_drift_free_water(const __grid_constant__ IntegrateArgs a, int nwater) {
   griddep_wait();
   if ((int)blockIdx.x < nwater)
-    kick_drift_body<NPT, 3, 3, true, CLOSE>(a, a.cls_begin[1], a.cls_begin[2], blockIdx.x);
+    kick_drift_body<NPT, 3, 3, true, CLOSE, LPW>(a, a.cls_begin[1], a.cls_begin[2], blockIdx.x);
   else
     kick_drift_body<NPT, 1, 0, false, CLOSE>(a, a.cls_begin[0], a.cls_begin[1], blockIdx.x - nwater);
 }
@@ -943,10 +998,25 @@ static int unit_grid(const IntegrateArgs& a) { return (a.u_end - a.u_begin + 127
 static bool free_and_water(const IntegrateArgs& a) {
   return a.settle && a.ncls == 2 && a.cls_na[0] == 1 && a.cls_nc[0] == 0 && a.cls_na[1] == 3 && a.cls_nc[1] == 3;
 }
+// Lanes per water: one lane each leaves SMs without a block below 148 x 128 waters; four
+// then shorten the pass (bound by one thread's chain) and still fit side by side.
+constexpr int kFewWaters = 148 * 128;
+
 template <bool NPT, bool CLOSE>
 static void launch_free_water(const IntegrateArgs& a, cudaStream_t st) {
-  const int nw = (a.cls_begin[2] - a.cls_begin[1] + 127) / 128, nf = (a.cls_begin[1] - a.cls_begin[0] + 127) / 128;
-  launch_pdl(k_drift_free_water<NPT, CLOSE>, dim3(nw + nf), dim3(128), 0, st, a, nw);
+  const int n = a.cls_begin[2] - a.cls_begin[1], nf = (a.cls_begin[1] - a.cls_begin[0] + 127) / 128;
+  if (n <= kFewWaters)
+    launch_pdl(k_drift_free_water<NPT, CLOSE, 4>, dim3((4 * n + 127) / 128 + nf), dim3(128), 0, st, a, (4 * n + 127) / 128);
+  else
+    launch_pdl(k_drift_free_water<NPT, CLOSE, 1>, dim3((n + 127) / 128 + nf), dim3(128), 0, st, a, (n + 127) / 128);
+}
+template <bool NPT, bool CLOSE>
+static void launch_water(const IntegrateArgs& a, cudaStream_t st) {
+  const int n = a.u_end - a.u_begin;
+  if (n <= kFewWaters)
+    launch_pdl(k_drift_water<NPT, CLOSE, 4>, dim3((4 * n + 127) / 128), dim3(128), 0, st, a);
+  else
+    launch_pdl(k_drift_water<NPT, CLOSE, 1>, dim3((n + 127) / 128), dim3(128), 0, st, a);
 }
 int drift_launches(const IntegrateArgs& a) { return free_and_water(a) ? 1 : a.ncls; }
 
@@ -959,7 +1029,7 @@ static void kick_drift_classes(const IntegrateArgs& a, cudaStream_t st) {
     constexpr int NA = decltype(na)::value, NC = decltype(nc)::value;
     if constexpr (NA == 3 && NC == 3) {
       if (x.settle) {
-        launch_pdl(k_kick_drift<NPT, 3, 3, true>, dim3(unit_grid(x)), dim3(128), 0, st, x);
+        launch_water<NPT, false>(x, st);
         return;
       }
     }
@@ -975,7 +1045,7 @@ void launch_close_kick_drift(const IntegrateArgs& a, cudaStream_t st) {
     constexpr int NA = decltype(na)::value, NC = decltype(nc)::value;
     if constexpr (NA == 3 && NC == 3) {
       if (x.settle) {
-        launch_pdl(k_close_kick_drift<3, 3, true>, dim3(unit_grid(x)), dim3(128), 0, st, x);
+        launch_water<false, true>(x, st);
         return;
       }
     }
