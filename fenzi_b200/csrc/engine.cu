@@ -584,23 +584,23 @@ static fz_status build_engine(fz_system* s, int device, void* stream) {
       if ((r = e->upload(&e->unit_terms, table)) || (r = e->upload(&e->unit_term_of, of))) return r;
     }
     for (int last = 0; last < 2; ++last) {
-    for (size_t k = 0; k < t.bond_k.size(); ++k) {
-      if (bin[k] != last) continue;
-      b.push_back(make_int2(t.bond[2 * k], t.bond[2 * k + 1]));
-      bp.push_back(make_float2((float)t.bond_k[k], (float)t.bond_r0[k]));
-    }
-    for (size_t k = 0; k < t.angle_k.size(); ++k) {
-      if (ain[k] != last) continue;
-      an.push_back(make_int4(t.angle[3 * k], t.angle[3 * k + 1], t.angle[3 * k + 2], 0));
-      ap.push_back(make_float2((float)t.angle_k[k], (float)t.angle_t0[k]));
-    }
-    for (size_t k = 0; k < t.excl_pairs.size() / 2; ++k)
-      if (xin[k] == last) x.push_back(make_int2(t.excl_pairs[2 * k], t.excl_pairs[2 * k + 1]));
-    if (!last) {
-      e->nbond_step = (int)b.size();
-      e->nangle_step = (int)an.size();
-      e->nexcl_step = (int)x.size();
-    }
+      for (size_t k = 0; k < t.bond_k.size(); ++k) {
+        if (bin[k] != last) continue;
+        b.push_back(make_int2(t.bond[2 * k], t.bond[2 * k + 1]));
+        bp.push_back(make_float2((float)t.bond_k[k], (float)t.bond_r0[k]));
+      }
+      for (size_t k = 0; k < t.angle_k.size(); ++k) {
+        if (ain[k] != last) continue;
+        an.push_back(make_int4(t.angle[3 * k], t.angle[3 * k + 1], t.angle[3 * k + 2], 0));
+        ap.push_back(make_float2((float)t.angle_k[k], (float)t.angle_t0[k]));
+      }
+      for (size_t k = 0; k < t.excl_pairs.size() / 2; ++k)
+        if (xin[k] == last) x.push_back(make_int2(t.excl_pairs[2 * k], t.excl_pairs[2 * k + 1]));
+      if (!last) {
+        e->nbond_step = (int)b.size();
+        e->nangle_step = (int)an.size();
+        e->nexcl_step = (int)x.size();
+      }
     }
     for (size_t k = 0; k < t.ub_k.size(); ++k) {
       u.push_back(make_int2(t.ub[2 * k], t.ub[2 * k + 1]));
