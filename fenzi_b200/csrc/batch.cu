@@ -368,15 +368,8 @@ static void batched_step_body(fz_batch* b, cudaStream_t st, bool open = true, bo
 static fz_status capture(fz_batch* b) {
   const int ns = (int)b->systems.size();
   fz_status r;
-  for (fz_system* s : b->systems) {
-    Engine* e = s->eng;
-    if (!e->forces_valid) {
-      FZ_CUDA(cudaMemsetAsync(e->facc, 0, 3 * sizeof(long long) * e->n, e->st));
-      e->forces(false);
-      e->forces_valid = true;
-    }
-    if ((r = e->check())) return r;
-  }
+  for (fz_system* s : b->systems)
+    if ((r = s->eng->check())) return r;
   if (!b->master) {
     FZ_CUDA(cudaStreamCreateWithFlags(&b->master, cudaStreamNonBlocking));
     FZ_CUDA(cudaEventCreateWithFlags(&b->ev_start, cudaEventDisableTiming));
@@ -429,6 +422,10 @@ extern "C" fz_status fz_batch_step(fz_batch* b, int nsteps) {
   FZ_CUDA(cudaSetDevice(b->dev));
   const int ns = (int)b->systems.size();
   fz_status r;
+  // a member whose positions were set since its last evaluation (set_state, set_positions,
+  // a restart file) starts from the forces of those positions, as fz_step does
+  for (fz_system* s : b->systems)
+    if ((r = s->eng->own_forces())) return r;
   if (!b->exec && (r = capture(b))) return r;
   // work queued on the systems' own streams precedes the batch
   for (int i = 0; i < ns; ++i) {

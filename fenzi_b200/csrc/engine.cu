@@ -916,11 +916,7 @@ extern "C" fz_status fz_step(fz_system* s, int nsteps) {
   if ((r = need_engine(s))) return r;
   if (nsteps < 0) return fail(FZ_ERR_ARG, "nsteps < 0");
   Engine* e = s->eng;
-  if (!e->forces_valid) {
-    FZ_CUDA(cudaMemsetAsync(e->facc, 0, 3 * sizeof(long long) * e->n, e->st));
-    e->forces(false);
-    e->forces_valid = true;
-  }
+  if ((r = e->own_forces())) return r;
   const fzk::IntegrateArgs ia = e->int_args();
   for (int k = 0; k < nsteps; ++k) {
     // a whole chunk in one graph launch when no velocity reassignment falls inside it

@@ -437,6 +437,15 @@ struct Engine {
     }
     mark(5);
   }
+  // the forces a step opens with: those the last step or evaluation left, or new ones where
+  // the positions have changed since
+  fz_status own_forces() {
+    if (forces_valid) return FZ_OK;
+    FZ_CUDA(cudaMemsetAsync(facc, 0, 3 * sizeof(long long) * n, st));
+    forces(false);
+    forces_valid = true;
+    return FZ_OK;
+  }
   // accumulates the events of one timed step: 0 start, 1..5 forces, 6 end
   void collect_step() {
     cudaEventSynchronize(ev[6]);

@@ -68,3 +68,37 @@ def test_batched_kernels_match_per_system_branches():
         assert np.array_equal(p1, p0)
         assert np.array_equal(v1, v0)
         assert np.array_equal(f1, f0)
+
+
+@pytest.mark.parametrize("kernels", ["1", "0"])
+@pytest.mark.parametrize("how", ["state", "positions", "checkpoint"])
+def test_members_given_new_positions_start_from_their_forces(how, kernels, monkeypatch, tmp_path):
+    """New positions for members of a batch that has already stepped: the next step opens
+    with the forces of those positions, as a system alone does (bit for bit)."""
+    monkeypatch.setenv("FZ_BATCH_KERNELS", kernels)
+    systems = gen_system.ensemble(nsys=3, seed=23, nw_min=216, nw_max=400)
+    alone = [_load(s, str(tmp_path / f"a{i}")) for i, s in enumerate(systems)]
+    mixed = [_load(s, str(tmp_path / f"b{i}")) for i, s in enumerate(systems)]
+    start = [(s.positions(), s.velocities()) for s in alone]
+    alone[0].SaveCheckpoint(str(tmp_path / "r"), "b")
+    b = fz.Batch(mixed)
+    b.step(7)
+    for s in alone:
+        s.SingleStep(7)
+    for i in (0, 2):  # the other member goes on
+        for s in (alone[i], mixed[i]):
+            if how == "checkpoint" and i == 0:
+                s.LoadCheckpoint(str(tmp_path / "r"), "b")
+            elif how == "positions":
+                s.set_positions(start[i][0])
+            else:
+                s.set_state_f32(start[i][0].astype(np.float32), start[i][1].astype(np.float32))
+    b.step(5)
+    for a, m in zip(alone, mixed):
+        a.SingleStep(5)
+        assert np.array_equal(a.positions(), m.positions())
+        assert np.array_equal(a.velocities(), m.velocities())
+        assert np.array_equal(a.forces_fixed(), m.forces_fixed())
+    b.close()
+    for s in alone + mixed:
+        s.close()
