@@ -292,6 +292,7 @@ struct Engine {
     a.n = n;
     for (int d = 0; d < 3; ++d) {
       a.K[d] = K[d];
+      a.set_scale(d, box_d[d]);
       a.B[d] = B[d];
       a.nb[d] = nbk[d];
       a.tw[d] = tw[d];

@@ -150,6 +150,19 @@ __device__ __forceinline__ void min_image_d(double* d, const SysParams& p) {
   d[2] -= (double)p.box.z * rint(d[2] / (double)p.box.z);
 }
 
+// Image of x in [-L/2, L/2).  One period is added or taken exactly (for L/2 <= |x| <= 2L the
+// FP32 difference has no rounding: Sterbenz, Floating-Point Computation (1974), 4.3.1), so
+// every image of an atom within that range gives the same number.
+__device__ __forceinline__ float wrap_coord(float x, float L, float invL) {
+  const float h = 0.5f * L;
+  if (!(x >= -h && x < h)) {
+    x = fmaf(-L, floorf(__fmul_rn(__fadd_rn(x, h), invL)), x);
+    if (x >= h) x -= L;
+    if (x < -h) x += L;
+  }
+  return x;
+}
+
 // periodic image code -> shift vector (code = (sx+1) + 3 (sy+1) + 9 (sz+1))
 __device__ __forceinline__ float3 shift_of(int code, const SysParams& p) {
   const int sx = code % 3 - 1, sy = (code / 3) % 3 - 1, sz = code / 9 - 1;

@@ -111,6 +111,11 @@ struct PmeArgs {
   const float4* pos4;
   int n;
   int K[3];
+  float scale_hi[3], scale_lo[3];  // K / L as the sum of two floats
+  void set_scale(int d, double L) {
+    scale_hi[d] = (float)(K[d] / L);
+    scale_lo[d] = (float)(K[d] / L - (double)scale_hi[d]);
+  }
   int B[3];     // brick edge per dimension
   int nb[3];    // bricks per dimension
   int* brick_of;     // [n]

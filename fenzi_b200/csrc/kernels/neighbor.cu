@@ -47,13 +47,9 @@ __device__ __forceinline__ void rb_bin_body(const RebuildArgs& A, int bid, int n
     atomicOr(status, ST_BAD_COORD);
     r.x = r.y = r.z = 0.f;
   }
-  r.x -= p.box.x * floorf((r.x + 0.5f * p.box.x) * p.inv_box.x);
-  r.y -= p.box.y * floorf((r.y + 0.5f * p.box.y) * p.inv_box.y);
-  r.z -= p.box.z * floorf((r.z + 0.5f * p.box.z) * p.inv_box.z);
-  // guard the rounding edge x == L/2
-  if (r.x >= 0.5f * p.box.x) r.x -= p.box.x;
-  if (r.y >= 0.5f * p.box.y) r.y -= p.box.y;
-  if (r.z >= 0.5f * p.box.z) r.z -= p.box.z;
+  r.x = wrap_coord(r.x, p.box.x, p.inv_box.x);
+  r.y = wrap_coord(r.y, p.box.y, p.inv_box.y);
+  r.z = wrap_coord(r.z, p.box.z, p.inv_box.z);
   pos4[a] = r;
   pos_build[a] = r;
   int cx = (int)((r.x + 0.5f * p.box.x) * p.inv_box.x * p.ncol[0]);

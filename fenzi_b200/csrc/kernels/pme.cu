@@ -30,14 +30,22 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
   return make_float2(fmaf(a.x, b.x, -__fmul_rn(a.y, b.y)), fmaf(a.x, b.y, __fmul_rn(a.y, b.x)));
 }
 
-// base grid point k0 and fraction t of coordinate x along a dimension of K points
-__device__ __forceinline__ int grid_base(float x, float invL, int K, float* t) {
-  float s = x * invL;
-  s -= floorf(s);
-  int k0 = (int)__fmul_rn(s, (float)K);
-  float f = fmaf(s, (float)K, -(float)k0);
-  if (k0 >= K) {
-    k0 -= K;
+// Base grid point k0 and fraction t of a coordinate along dimension d of K points.  The
+// coordinate is brought into the box first, exactly, and the fraction is x K / L - k0 from a
+// scale held in two floats: it does not depend on which image of an atom a caller holds (a
+// step reads the positions its drift made, a force call those that a rebuild has wrapped
+// since), and its error is its own rounding.  Explicit operations: every kernel must find the
+// same point (a brick's atoms are binned by one kernel and spread by another).
+__device__ __forceinline__ int grid_base(const PmeArgs& a, int d, float x, int K, float* t) {
+  const float L = d == 0 ? a.p.box.x : (d == 1 ? a.p.box.y : a.p.box.z);
+  const float invL = d == 0 ? a.p.inv_box.x : (d == 1 ? a.p.inv_box.y : a.p.inv_box.z);
+  x = wrap_coord(x, L, invL);
+  const float k = floorf(__fmul_rn(x, a.scale_hi[d]));
+  float f = fmaf(x, a.scale_lo[d], fmaf(x, a.scale_hi[d], -k));
+  int k0 = (int)k;
+  k0 += k0 < 0 ? K : 0;
+  if (k0 < 0 || k0 >= K) {  // no position of this box (beyond FP32's resolution of it)
+    k0 = 0;
     f = 0.f;
   }
   *t = f;
@@ -85,9 +93,9 @@ __device__ __forceinline__ void pme_bin_body(const PmeArgs& a, int bid, int nbid
   if (i >= a.n) return;
   const float4 r = a.pos4[i];
   float t;
-  const int kx = grid_base(r.x, a.p.inv_box.x, a.K[0], &t);
-  const int ky = grid_base(r.y, a.p.inv_box.y, a.K[1], &t);
-  const int kz = grid_base(r.z, a.p.inv_box.z, a.K[2], &t);
+  const int kx = grid_base(a, 0, r.x, a.K[0], &t);
+  const int ky = grid_base(a, 1, r.y, a.K[1], &t);
+  const int kz = grid_base(a, 2, r.z, a.K[2], &t);
   const int b = ((kz / a.B[2]) * a.nb[1] + ky / a.B[1]) * a.nb[0] + kx / a.B[0];
   a.brick_of[i] = b;
   // warp-aggregated increment: one atomic per distinct brick in the warp
@@ -189,9 +197,9 @@ __device__ __forceinline__ void pme_spread_body(const PmeArgs& a, int bid, int n
   for (int idx = s0 + threadIdx.x; idx < s1; idx += blockDim.x) {
     const float4 r = a.pos4[a.brick_atoms[idx]];
     float tx, ty, tz, wx[4], wy[4], wz[4];
-    const int kx = grid_base(r.x, a.p.inv_box.x, Kx, &tx) - ox;
-    const int ky = grid_base(r.y, a.p.inv_box.y, Ky, &ty) - oy;
-    const int kz = grid_base(r.z, a.p.inv_box.z, Kz, &tz) - oz;
+    const int kx = grid_base(a, 0, r.x, Kx, &tx) - ox;
+    const int ky = grid_base(a, 1, r.y, Ky, &ty) - oy;
+    const int kz = grid_base(a, 2, r.z, Kz, &tz) - oz;
     bsp4(tx, wx, nullptr);
     bsp4(ty, wy, nullptr);
     bsp4(tz, wz, nullptr);
@@ -254,9 +262,9 @@ __global__ void __launch_bounds__(256) k_pme_spread_atoms(PmeArgs a) {
   const int Kx = a.K[0], Ky = a.K[1], Kz = a.K[2];
   const float4 r = a.pos4[i];
   float tx, ty, tz, wx[4], wy[4], wz[4];
-  const int kx = grid_base(r.x, a.p.inv_box.x, Kx, &tx);
-  const int ky = grid_base(r.y, a.p.inv_box.y, Ky, &ty);
-  const int kz = grid_base(r.z, a.p.inv_box.z, Kz, &tz);
+  const int kx = grid_base(a, 0, r.x, Kx, &tx);
+  const int ky = grid_base(a, 1, r.y, Ky, &ty);
+  const int kz = grid_base(a, 2, r.z, Kz, &tz);
   bsp4(tx, wx, nullptr);
   bsp4(ty, wy, nullptr);
   bsp4(tz, wz, nullptr);
@@ -529,9 +537,9 @@ __device__ __forceinline__ void pme_gather_atoms_body(const PmeArgs& a, int bid,
   const int Kx = a.K[0], Ky = a.K[1], Kz = a.K[2];
   const float4 r = a.pos4[i];
   float tx, ty, tz, wx[4], wy[4], wz[4], dx[4], dy[4], dz[4];
-  const int kx = grid_base(r.x, a.p.inv_box.x, Kx, &tx);
-  const int ky = grid_base(r.y, a.p.inv_box.y, Ky, &ty);
-  const int kz = grid_base(r.z, a.p.inv_box.z, Kz, &tz);
+  const int kx = grid_base(a, 0, r.x, Kx, &tx);
+  const int ky = grid_base(a, 1, r.y, Ky, &ty);
+  const int kz = grid_base(a, 2, r.z, Kz, &tz);
   bsp4(tx, wx, dx);
   bsp4(ty, wy, dy);
   bsp4(tz, wz, dz);
@@ -612,9 +620,9 @@ __device__ __forceinline__ void pme_gather_body(const PmeArgs& a, int bid, int n
     const int i = a.brick_atoms[idx];
     const float4 r = a.pos4[i];
     float tx, ty, tz, wx[4], wy[4], wz[4], dx[4], dy[4], dz[4];
-    const int kx = grid_base(r.x, a.p.inv_box.x, Kx, &tx) - ox;
-    const int ky = grid_base(r.y, a.p.inv_box.y, Ky, &ty) - oy;
-    const int kz = grid_base(r.z, a.p.inv_box.z, Kz, &tz) - oz;
+    const int kx = grid_base(a, 0, r.x, Kx, &tx) - ox;
+    const int ky = grid_base(a, 1, r.y, Ky, &ty) - oy;
+    const int kz = grid_base(a, 2, r.z, Kz, &tz) - oz;
     bsp4(tx, wx, dx);
     bsp4(ty, wy, dy);
     bsp4(tz, wz, dz);
@@ -1238,9 +1246,9 @@ __device__ __noinline__ void pme_box_body(const PmeArgs& a) {
   for (int i = tid; i < a.n; i += kBoxThreads) {
     const float4 r = a.pos4[i];
     float tx, ty, tz, wx[4], wy[4], wz[4];
-    const int kx = grid_base(r.x, a.p.inv_box.x, N, &tx);
-    const int ky = grid_base(r.y, a.p.inv_box.y, N, &ty);
-    const int kz = grid_base(r.z, a.p.inv_box.z, N, &tz);
+    const int kx = grid_base(a, 0, r.x, N, &tx);
+    const int ky = grid_base(a, 1, r.y, N, &ty);
+    const int kz = grid_base(a, 2, r.z, N, &tz);
     bsp4(tx, wx, nullptr);
     bsp4(ty, wy, nullptr);
     bsp4(tz, wz, nullptr);
@@ -1355,9 +1363,9 @@ __device__ __noinline__ void pme_box_body(const PmeArgs& a) {
   for (int i = tid; i < n; i += kBoxThreads) {
     const float4 r = a.pos4[i];
     float tx, ty, tz, wx[4], wy[4], wz[4], dx[4], dy[4], dz[4];
-    const int kx = grid_base(r.x, a.p.inv_box.x, N, &tx);
-    const int ky = grid_base(r.y, a.p.inv_box.y, N, &ty);
-    const int kz = grid_base(r.z, a.p.inv_box.z, N, &tz);
+    const int kx = grid_base(a, 0, r.x, N, &tx);
+    const int ky = grid_base(a, 1, r.y, N, &ty);
+    const int kz = grid_base(a, 2, r.z, N, &tz);
     bsp4(tx, wx, dx);
     bsp4(ty, wy, dy);
     bsp4(tz, wz, dz);

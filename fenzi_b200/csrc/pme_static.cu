@@ -180,6 +180,7 @@ extern "C" fz_status fz_pme_reciprocal_static(int device, void* stream, const fl
   a.n = n;
   for (int d = 0; d < 3; ++d) {
     a.K[d] = K[d];
+    a.set_scale(d, box[d]);
     a.B[d] = brick_edge(K[d]);
     a.nb[d] = K[d] / a.B[d];
     a.p.K[d] = K[d];

@@ -1,9 +1,9 @@
-"""The rigid waters' own terms, evaluated by the integrator's pass in a step and by the
-bonded kernel in a force call: the forces a step leaves behind are those of a force call
-at its positions, bit for bit (all sums are integers), as long as the last step has not
-wrapped positions (no rebuild).  Unit counts around a 128-thread block, with chains (two
-unit classes in one launch) and without; the terms themselves are checked against the
-oracle in test_gpu_terms.py."""
+"""The forces a step leaves behind against a force call at its positions, bit for bit (all sums
+are integers).  In a step the rigid waters' own terms come from the integrator's pass, and PME
+and the other bonded terms read the positions before a rebuild wraps them; a force call has
+every term from its own kernel and reads the wrapped ones.  Steps that rebuild are among those
+compared.  With chains (two unit classes in one launch) and without; the terms themselves are
+checked against the oracle in test_gpu_terms.py."""
 import numpy as np
 import pytest
 
@@ -13,20 +13,40 @@ from tests.helpers import system
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nw,chains", [(127, 0), (128, 2), (129, 0), (400, 3)])
-def test_forces_left_by_a_step_equal_a_force_call(nw, chains):
+def _start(nw, chains, T=300.0):
     kw = {} if chains == 0 else dict(chain_len=10)
     _, path = system(f"wt_{nw}_{chains}", name="custom", nw=nw, nchains=chains, rc=6.5, ron=5.0, seed=nw, **kw)
     s = fz.FenZi.ReadInput(path).LoadSystem()
     s.InitMem(0)
-    s.InitVelocity(T=100.0, seed=5)
-    s.SingleStep(1)  # the list rebuild of the start
-    for n in (1, 2, 3):
+    s.InitVelocity(T=T, seed=5)
+    return s
+
+
+@pytest.mark.parametrize("nw,chains", [(127, 0), (128, 2), (129, 0), (400, 3)])
+def test_forces_left_by_a_step_equal_a_force_call(nw, chains):
+    s = _start(nw, chains)
+    at_rebuild = 0
+    for n in (1, 2, 3) + (1,) * 20:
+        s.SingleStep(n - 1)
         before = s.counters()["rebuilds"]
-        s.SingleStep(n)
+        s.SingleStep(1)
+        at_rebuild += s.counters()["rebuilds"] > before
         left = s.forces_fixed()
         s.ComputeAccelGPU()
-        if s.counters()["rebuilds"] == before:
-            assert np.array_equal(left, s.forces_fixed())
-    assert s.counters()["rebuilds"] < 4
+        assert np.array_equal(left, s.forces_fixed())
+    assert at_rebuild >= 2
     s.close()
+
+
+@pytest.mark.parametrize("nw,chains", [(400, 0), (900, 2)])
+def test_a_run_does_not_depend_on_its_print_interval(nw, chains):
+    a, b = _start(nw, chains), _start(nw, chains)
+    for k in range(40):
+        a.SingleStep(3)
+        b.SingleStep(3)
+        b.EvalProps()
+    assert b.counters()["rebuilds"] > 10
+    assert np.array_equal(a.positions(), b.positions())
+    assert np.array_equal(a.velocities(), b.velocities())
+    for s in (a, b):
+        s.close()
