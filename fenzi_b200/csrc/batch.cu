@@ -98,6 +98,7 @@ struct fz_batch {
   cudaStream_t master = nullptr;
   cudaEvent_t ev_start = nullptr, ev_master = nullptr;
   std::vector<cudaEvent_t> ev_done;
+  std::vector<unsigned long long> stamps;  // Engine::args_stamp of each member at the capture
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   // batched kernels only: a graph of `chunk` consecutive steps (one launch per chunk)
@@ -422,6 +423,20 @@ extern "C" fz_status fz_batch_step(fz_batch* b, int nsteps) {
   FZ_CUDA(cudaSetDevice(b->dev));
   const int ns = (int)b->systems.size();
   fz_status r;
+  // the graph holds the members' kernel arguments by value: captured again when a member
+  // has been uploaded anew or has another box
+  std::vector<unsigned long long> stamps;
+  for (int i = 0; i < ns; ++i) {
+    const Engine* e = b->systems[i]->eng;
+    if (!e || e->dev != b->dev)
+      return fail(FZ_ERR_STATE, "fz_batch_step: system " + std::to_string(i) + " is no longer on the batch's device");
+    stamps.push_back(e->args_stamp);
+  }
+  if (b->exec && stamps != b->stamps) {
+    FZ_CUDA(cudaStreamSynchronize(b->master));
+    b->drop_graph();
+  }
+  b->stamps = stamps;
   // a member whose positions were set since its last evaluation (set_state, set_positions,
   // a restart file) starts from the forces of those positions, as fz_step does
   for (fz_system* s : b->systems)

@@ -746,6 +746,7 @@ constexpr double kPatm = 68558.64100846418;     // kcal/mol/A^3 -> atm (src/cell
 // value to the kernels, the column search reach, and the PME influence tables.
 fz_status set_box(Engine* e, double L) {
   fzk::SysParams& p = e->p;
+  e->args_stamp = Engine::next_stamp();
   for (int d = 0; d < 3; ++d) e->box_d[d] = L * e->ratio[d];
   const double lmin = std::min(e->box_d[0], std::min(e->box_d[1], e->box_d[2]));
   if (e->cutoff >= 0.5 * lmin) return fail(FZ_ERR_STATE, "barostat: box shrank below twice the cutoff");
@@ -1084,6 +1085,7 @@ extern "C" fz_status fz_set_barostat(fz_system* s, int enable, double pref_atm, 
   Engine* e = s->eng;
   if (enable && !(pmass > 0.0)) return fail(FZ_ERR_ARG, "fz_set_barostat: piston mass must be positive");
   e->drop_graph();
+  e->args_stamp = Engine::next_stamp();
   if (!enable) {
     e->npt = false;
     e->p.skin_half2 = e->skin_half2_nve;

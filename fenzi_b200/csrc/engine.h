@@ -2,6 +2,7 @@
 // pieces queued on its stream.  Shared by the single-system C ABI (engine.cu) and the
 // batched ensemble / serving loop (batch.cu).
 #pragma once
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -92,6 +93,13 @@ struct Engine {
   float2* tw[3] = {nullptr, nullptr, nullptr};
   float *gfac[3] = {nullptr, nullptr, nullptr}, *f2[3] = {nullptr, nullptr, nullptr};
   float gscale = 0.f;
+  // which kernel arguments this engine hands out: another number in every engine and after
+  // every change of the box or of the list tests, so that a batch knows when its own are old
+  unsigned long long args_stamp = next_stamp();
+  static unsigned long long next_stamp() {
+    static std::atomic<unsigned long long> last{0};
+    return ++last;
+  }
   // run state
   bool forces_valid = false;
   long long step = 0;

@@ -102,3 +102,36 @@ def test_members_given_new_positions_start_from_their_forces(how, kernels, monke
     b.close()
     for s in alone + mixed:
         s.close()
+
+
+@pytest.mark.parametrize("kernels", ["1", "0"])
+def test_batch_follows_members_of_another_box_or_uploaded_anew(kernels, monkeypatch, tmp_path):
+    """The graph of a batch holds its members' boxes and device addresses.  A restart file of
+    another box and a new upload change them between two calls: the members still move as
+    they do alone, bit for bit."""
+    monkeypatch.setenv("FZ_BATCH_KERNELS", kernels)
+    systems = gen_system.ensemble(nsys=3, seed=31, nw_min=400, nw_max=500)
+    piston = _load(systems[0], str(tmp_path / "p"))
+    piston.set_barostat(True, pref_atm=1.0, pmass=1e-6)
+    piston.SingleStep(20)
+    piston.SaveCheckpoint(str(tmp_path / "r"), "b")
+    assert abs(piston.EvalProps()["box"][0] / systems[0].box[0] - 1.0) > 1e-5
+    alone = [_load(s, str(tmp_path / f"a{i}")) for i, s in enumerate(systems)]
+    mixed = [_load(s, str(tmp_path / f"b{i}")) for i, s in enumerate(systems)]
+    b = fz.Batch(mixed)
+    b.step(6)
+    for s in alone:
+        s.SingleStep(6)
+    for s in (alone[0], mixed[0]):
+        s.LoadCheckpoint(str(tmp_path / "r"), "b")
+    for s in (alone[1], mixed[1]):
+        s.InitMem(0)
+        s.InitVelocity(T=200.0, seed=4)
+    b.step(6)
+    for a, m in zip(alone, mixed):
+        a.SingleStep(6)
+        assert np.array_equal(a.positions(), m.positions())
+        assert np.array_equal(a.velocities(), m.velocities())
+    b.close()
+    for s in alone + mixed + [piston]:
+        s.close()
