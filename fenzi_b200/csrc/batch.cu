@@ -517,23 +517,6 @@ struct Job {
   std::vector<double> pos;
 };
 
-// Device bytes of one uploaded system, an upper estimate of build_engine's allocations:
-// ~164 B per atom of atom, slot, PME-binning and transfer arrays, the per-block pair lists, masks
-// and work items (~0.5 B per atom per unit of list capacity, the capacity estimated as
-// build_engine does), the PME grids and charge staging (~24 B per grid point), and 8 MiB
-// of fixed overhead.
-size_t engine_bytes_estimate(const fz_system* s) {
-  const double n = (double)s->top.n;
-  const double V = s->cfg.box[0] * s->cfg.box[1] * s->cfg.box[2];
-  const double rho = n / V;
-  const double K3 = (double)s->cfg.pme_grid[0] * s->cfg.pme_grid[1] * s->cfg.pme_grid[2];
-  const double R = std::max(s->cfg.pairlistdist, s->cfg.cutoff);
-  const double a = 1.4 * std::cbrt(32.0 / rho);
-  const double vm = a * a * a + 6 * a * a * R + 3 * M_PI * a * R * R + 4.0 / 3.0 * M_PI * R * R * R;
-  const double ocap = std::max(256.0, 1.25 * rho * vm);
-  return (size_t)(n * (164.0 + 0.5 * ocap) + 24.0 * K3) + ((size_t)8 << 20);
-}
-
 }  // namespace
 
 struct fz_server {
@@ -673,7 +656,7 @@ void fz_server::run() {
 
 extern "C" fz_status fz_server_estimate_bytes(const fz_system* sys, double* out) {
   if (!sys || !out) return fail(FZ_ERR_ARG, "null argument");
-  *out = (double)engine_bytes_estimate(sys);
+  *out = (double)device_bytes(sys);
   return FZ_OK;
 }
 
@@ -703,7 +686,7 @@ extern "C" fz_status fz_server_submit(fz_server* sv, fz_system* sys, long long n
   std::unique_ptr<Job> j(new Job());
   j->sys = sys;
   j->nsteps = nsteps;
-  j->est_bytes = engine_bytes_estimate(sys);
+  j->est_bytes = device_bytes(sys);
   std::lock_guard<std::mutex> lock(sv->mu);
   if (sv->stop) return fail(FZ_ERR_STATE, "fz_server_submit: server is stopping");
   j->id = sv->next_id++;

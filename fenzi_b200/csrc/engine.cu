@@ -204,6 +204,111 @@ static fz_status autotune(Engine* e) {
   return e->check();
 }
 
+// column grid of the neighbour sort, sorted slots and per-block list capacity of a system
+struct ListShape {
+  int ncx, ncy, nslots, ocap;
+  double col_a;
+};
+static ListShape list_shape(const fz_config& c, int n) {
+  const double rho = n / (c.box[0] * c.box[1] * c.box[2]);
+  // column cross-section: a x a with a^3 holding `col_atoms` atoms (32: one sorted
+  // block is a near-cube; smaller values make narrower, taller blocks).  16: a block
+  // is two near-cubes stacked in z, so each 16-atom i-group is a compact cube and
+  // fewer pairs of its tiles fall outside the cutoff.  Measured (us per step, 1,000
+  // steps): 230,400 atoms 421 (32) / 413-418 (16); 17,280 atoms 85.9 / 83.7; 256
+  // boxes 1.655 / 1.608 ms.
+  double col_atoms = 16.0;
+  if (const char* v = std::getenv("FZ_COL_ATOMS")) col_atoms = std::min(64.0, std::max(8.0, std::atof(v)));
+  const double a = std::cbrt(col_atoms / rho);
+  int ncx = std::max(1, (int)std::floor(c.box[0] / a)), ncy = std::max(1, (int)std::floor(c.box[1] / a));
+  while ((double)n / (ncx * ncy) > fzk::kColCap / 2 && (ncx < 4096 && ncy < 4096)) {
+    ncx *= 2;
+    ncy *= 2;
+  }
+  // per-block list capacity: atoms within rlist of a block box (Minkowski volume of a
+  // box 1.4 a wide and 1.4 h tall, h the mean height of 32 atoms in a column), with
+  // room for blocks that see all their neighbours at higher index
+  const double ab = 1.4 * a, hb = 1.4 * 32.0 / (rho * a * a), R = std::max(c.pairlistdist, c.cutoff);
+  const double vm = ab * ab * hb + 2 * R * (ab * ab + 2 * ab * hb) + M_PI * R * R * (2 * ab + hb) +
+                    4.0 / 3.0 * M_PI * R * R * R;
+  ListShape s;
+  s.ncx = ncx;
+  s.ncy = ncy;
+  s.nslots = ((n + 32 * ncx * ncy + 64 + 31) / 32) * 32;
+  s.ocap = (int)std::ceil(std::max(256.0, 1.25 * rho * vm) / 32.0) * 32;
+  s.col_a = a;
+  return s;
+}
+
+// Device bytes of one uploaded system: build_engine's allocations, each as cudaMalloc rounds
+// it (2 MiB from 1 MiB on, else 512 bytes out of shared 2 MiB pieces), and 12 MiB for its
+// graphs (measured: 8 to 11) and the rest.  More only where a list outgrows its capacity and
+// is made anew twice as large.  Against the memory in use after 200 steps: 648 atoms 14.2 MB of
+// 12.6, 6,000 29.8 of 18.9, 17,280 57.0 of 54.5, 230,400 520 of 505.
+size_t device_bytes(const fz_system* sys) {
+  const Topology& t = sys->top;
+  const fz_config& c = sys->cfg;
+  const ListShape s = list_shape(c, t.n);
+  const size_t n = t.n, ns = s.nslots, blk = ns / 32, grp = blk * fzk::kNG, tiles = s.ocap / 32;
+  size_t total = (size_t)12 << 20;
+  auto add = [&](size_t bytes) {
+    const size_t unit = bytes >= ((size_t)1 << 20) ? (size_t)2 << 20 : 512;
+    total += (bytes + unit - 1) / unit * unit;
+  };
+  // atoms: positions (current, built, pruned, drifted), velocities; forces, transfers; indices
+  for (int k = 0; k < 5; ++k) add(16 * n);
+  for (int k = 0; k < 2; ++k) add(24 * n);
+  for (int k = 0; k < 6; ++k) add(4 * n);  // type, slot, column, brick, brick order, exclusion offset
+  size_t units = n, xmax = 1;
+  if (c.consfix_nseg == 0)  // (the atoms of a fixed cluster are units of their own)
+    for (const Cluster& cl : t.clusters) units -= cl.na - 1;
+  add(16 * units);
+  add(16 * units);
+  add(4 * units);
+  add(4 * units);
+  for (size_t i = 0; i < n; ++i) xmax = std::max<size_t>(xmax, t.excl_off[i + 1] - t.excl_off[i]);
+  add(4 * t.excl_idx.size());
+  if (c.consharm) {
+    add(4 * n);
+    add(4 * n);
+  }
+  // slots, blocks, i-groups
+  add(16 * ns);
+  for (int k = 0; k < 5; ++k) add(4 * ns);
+  add(8 * ns);
+  add(4 * ns * xmax);
+  for (int k = 0; k < 2; ++k) add(16 * blk);
+  for (int k = 0; k < 2; ++k) add(4 * blk);
+  add(4 * blk * s.ocap);
+  add(4 * grp * s.ocap);
+  add(4 * grp);
+  add(4 * grp * tiles);
+  add(4 * grp * tiles * fzk::kIG);
+  add(8 * grp * (tiles + 1));
+  for (int k = 0; k < 3; ++k) add(4 * ((size_t)s.ncx * s.ncy + 1));
+  // terms and their parameters
+  for (size_t m : {t.bond_k.size(), t.ub_k.size()}) {
+    add(8 * m);
+    add(8 * m);
+  }
+  for (size_t m : {t.angle_k.size(), t.impr_k.size(), t.dihe_k.size()}) {
+    add(16 * m);
+    add(16 * m);
+  }
+  add(4 * t.excl_pairs.size());
+  add(4 * t.p14_pairs.size());
+  // PME
+  const size_t Kx = c.pme_grid[0], Ky = c.pme_grid[1], Kz = c.pme_grid[2];
+  const int K[3] = {c.pme_grid[0], c.pme_grid[1], c.pme_grid[2]};
+  if (!(fft_size_ok(K[0]) && fft_size_ok(K[1]) && fft_size_ok(K[2]))) return total;  // refused at upload
+  size_t nbr = 1;
+  for (const auto& b : brick_candidates(K)) nbr = std::max(nbr, (Kx / b[0]) * (Ky / b[1]) * (Kz / b[2]));
+  for (int k = 0; k < 3; ++k) add(4 * (nbr + 1));
+  add(4 * Kx * Ky * Kz);
+  add(8 * Kz * Ky * (Kx / 2 + 1));
+  return total;
+}
+
 static fz_status build_engine(fz_system* s, int device, void* stream) {
   const Topology& t = s->top;
   const fz_config& c = s->cfg;
@@ -250,20 +355,9 @@ static fz_status build_engine(fz_system* s, int device, void* stream) {
   if (rc >= 0.5 * lmin) return fail(FZ_ERR_ARG, "cutoff must be below half the smallest box edge");
   const double V = c.box[0] * c.box[1] * c.box[2];
   const double rho = n / V;
-  // column cross-section: a x a with a^3 holding `col_atoms` atoms (32: one sorted
-  // block is a near-cube; smaller values make narrower, taller blocks).  16: a block
-  // is two near-cubes stacked in z, so each 16-atom i-group is a compact cube and
-  // fewer pairs of its tiles fall outside the cutoff.  Measured (us per step, 1,000
-  // steps): 230,400 atoms 421 (32) / 413-418 (16); 17,280 atoms 85.9 / 83.7; 256
-  // boxes 1.655 / 1.608 ms.
-  double col_atoms = 16.0;
-  if (const char* v = std::getenv("FZ_COL_ATOMS")) col_atoms = std::min(64.0, std::max(8.0, std::atof(v)));
-  const double a = std::cbrt(col_atoms / rho);
-  int ncx = std::max(1, (int)std::floor(c.box[0] / a)), ncy = std::max(1, (int)std::floor(c.box[1] / a));
-  while ((double)n / (ncx * ncy) > fzk::kColCap / 2 && (ncx < 4096 && ncy < 4096)) {
-    ncx *= 2;
-    ncy *= 2;
-  }
+  const ListShape ls = list_shape(c, n);
+  const double a = ls.col_a;
+  const int ncx = ls.ncx, ncy = ls.ncy;
   p.ncol[0] = ncx;
   p.ncol[1] = ncy;
   e->ncol = ncx * ncy;
@@ -281,7 +375,7 @@ static fz_status build_engine(fz_system* s, int device, void* stream) {
   e->L_build = e->L_prune = c.box[0];
   e->pmass = c.pmass;
   e->pref_atm = c.pref;
-  e->nslots = ((n + 32 * e->ncol + 64 + 31) / 32) * 32;
+  e->nslots = ls.nslots;
   p.nslots = e->nslots;
   if (e->nslots >= (1 << 26)) return fail(FZ_ERR_CAPACITY, "system too large: sorted slots exceed 2^26");
   for (int d = 0; d < 3; ++d) {
@@ -297,13 +391,7 @@ static fz_status build_engine(fz_system* s, int device, void* stream) {
     p.K[d] = e->K[d];
   }
   if (const char* v = std::getenv("FZ_PME_GATHER")) e->gather_mode = std::max(0, std::min(3, std::atoi(v)));
-  // per-block list capacity: atoms within rlist of a block box (Minkowski volume of a
-  // box 1.4 a wide and 1.4 h tall, h the mean height of 32 atoms in a column), with
-  // room for blocks that see all their neighbours at higher index
-  const double ab = 1.4 * a, hb = 1.4 * 32.0 / (rho * a * a), R = plist;
-  const double vm = ab * ab * hb + 2 * R * (ab * ab + 2 * ab * hb) + M_PI * R * R * (2 * ab + hb) +
-                    4.0 / 3.0 * M_PI * R * R * R;
-  e->ocap = (int)std::ceil(std::max(256.0, 1.25 * rho * vm) / 32.0) * 32;
+  e->ocap = ls.ocap;
   e->mask_cap = (e->nslots / 32) * fzk::kNG * (e->ocap / 32);
   {
     // inner-list buffer: a larger delta prunes less often but leaves more pairs.

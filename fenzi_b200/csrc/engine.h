@@ -611,5 +611,7 @@ struct Engine {
 // moves an engine to the box with x edge L (aspect ratios kept): kernel parameters,
 // column reach and PME influence tables (engine.cu)
 fz_status set_box(Engine* e, double L);
+// upper estimate of an uploaded system's device memory (engine.cu)
+size_t device_bytes(const fz_system* sys);
 
 }  // namespace fz

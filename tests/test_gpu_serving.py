@@ -71,3 +71,25 @@ def test_server_rejects_job_above_budget(job_paths):
     assert ei.value.code == 4  # FZ_ERR_CAPACITY
     assert server.info(k)["state"] == "failed"
     server.close()
+
+
+@pytest.mark.parametrize("kw", [dict(name="custom", nw=216, rc=9.0, ron=7.5), dict(name="custom", nw=2000, rc=9.0, ron=7.5),
+                                dict(name="chain17k"), dict(name="large230k")], ids=["648", "6000", "17280", "230400"])
+def test_estimate_is_above_the_memory_in_use(kw, tmp_path):
+    """The admission estimate against the device memory that an upload and 200 steps take
+    (their graph among it): never below, and at most a half and 16 MB above."""
+    import torch
+    path = gen_system.write(gen_system.build(**kw), str(tmp_path))
+    warm = fz.FenZi.ReadInput(path).LoadSystem()
+    est = fz.Server.estimate_bytes(warm)
+    warm.InitMem(0)  # what the first system of a process costs is not the system's
+    warm.SingleStep(1)
+    free = torch.cuda.mem_get_info()[0]
+    s = fz.FenZi.ReadInput(path).LoadSystem()
+    s.InitMem(0)
+    s.InitVelocity(T=100.0, seed=2)
+    s.SingleStep(200)
+    used = free - torch.cuda.mem_get_info()[0]
+    assert used <= est <= 1.5 * used + 16e6
+    s.close()
+    warm.close()
