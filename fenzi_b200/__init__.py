@@ -91,7 +91,7 @@ EXPORTS = ["fz_last_error", "fz_version", "fz_read_input", "fz_load_system", "fz
            "fz_get_forces_fixed", "fz_set_state_f32", "fz_get_state_f32", "fz_get_counters", "fz_get_launch_shapes", "fz_sync",
            "fz_stream", "fz_set_stage_timing", "fz_get_stage_times", "fz_measure_fp32_peak",
            "fz_pme_reciprocal_static", "fz_batch_create", "fz_batch_add", "fz_batch_step", "fz_batch_free",
-           "fz_set_barostat", "fz_get_virial", "fz_batch_remove", "fz_batch_size", "fz_server_create",
+           "fz_set_barostat", "fz_get_virial", "fz_batch_remove", "fz_batch_size", "fz_batch_launches", "fz_server_create",
            "fz_server_submit", "fz_server_info", "fz_server_wait", "fz_server_positions", "fz_server_stats",
            "fz_server_free", "fz_server_estimate_bytes", "fz_checkpoint_save", "fz_checkpoint_load",
            "fz_dcd_open", "fz_dcd_write", "fz_dcd_close", "fz_minimize"]
@@ -153,6 +153,7 @@ def lib():
             "fz_get_virial": ([vp, dp], C.c_int),
             "fz_batch_remove": ([vp, vp], C.c_int),
             "fz_batch_size": ([vp, C.POINTER(C.c_int)], C.c_int),
+            "fz_batch_launches": ([vp, C.POINTER(C.c_longlong)], C.c_int),
             "fz_server_create": ([C.c_int, C.c_double, C.c_int, C.c_int, C.POINTER(vp)], C.c_int),
             "fz_server_submit": ([vp, vp, C.c_longlong, C.POINTER(C.c_int)], C.c_int),
             "fz_server_info": ([vp, C.c_int, C.POINTER(JobInfo)], C.c_int),
@@ -410,6 +411,12 @@ class Batch:
 
     def step(self, nsteps=1):
         _check(lib().fz_batch_step(self.h, int(nsteps)))
+
+    def launches_per_step(self) -> int:
+        """Kernels that one step of the batch launches (0 before its first step)."""
+        out = C.c_longlong()
+        _check(lib().fz_batch_launches(self.h, C.byref(out)))
+        return out.value
 
     def close(self):
         if self.h:

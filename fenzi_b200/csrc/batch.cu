@@ -189,9 +189,10 @@ static bool batched_kernels_ok(const fz_batch* b) {
 }
 
 // Members from which the PME of small grids is a block per member.  us a step, blocks /
-// launches: 6 boxes of 216 to 2,000 waters 137 / 137, 12: 175 / 194, 24: 236 / 255, 48: 342
-// / 365, 96: 583 / 632; 24 of 1,500 to 2,000: 293 / 307; 64 of 216 to 500: 225 / 240.  The
-// numbers are the same either way.
+// launches: 6 boxes of 216 to 2,000 waters 137 / 137, 8: 167 / 179, 16: 212 / 227, 24: 236 /
+// 255, 48: 342 / 365, 96: 583 / 632; 8 of 216: 125 / 128, 8 of 1,500 to 2,000: 181 / 192; 64 of
+// 216 to 500: 225 / 240.  (8 equal members on a grid much finer than usual, 3,000 atoms on
+// 36^3, lose: 102 / 95; 16 of them gain: 115 / 136.)  The numbers are the same either way.
 constexpr int kBoxMembers = 8;
 
 static void add_blocks(std::vector<int4>& tab, int arg, int nblocks) {
@@ -485,6 +486,16 @@ extern "C" fz_status fz_batch_step(fz_batch* b, int nsteps) {
     if (b->pinned_status[i] && (r = b->systems[i]->eng->check()))
       return fail(r, "system " + std::to_string(i) + " of the batch: " + last_error_text());
   b->steps += nsteps;
+  return FZ_OK;
+}
+
+extern "C" fz_status fz_batch_launches(fz_batch* b, long long* out) {
+  if (!b || !out) return fail(FZ_ERR_ARG, "null argument");
+  *out = 0;
+  if (!b->exec) return FZ_OK;
+  if (b->bk) *out = b->bk->launches;
+  else
+    for (const fz_system* s : b->systems) *out += s->eng ? s->eng->graph_step_launches() : 0;
   return FZ_OK;
 }
 

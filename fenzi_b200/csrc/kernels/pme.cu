@@ -1182,12 +1182,14 @@ __global__ void __launch_bounds__(kPlaneThreads) k_fft_yx_plane_b(const PmeArgs*
 // (odd, to spread rows over the banks).  A thread takes a whole line through its DFT in
 // registers (the stages, radices and row pairing of the plane and z kernels, so the
 // potentials are the same numbers) and puts it back where it was; the z pass does both
-// directions with the influence function between them.
-// What it replaces: ten launches, then three for every grid size among the members, each
+// directions with the influence function between them.  Registers hold the line up to N = 25;
+// above that some of it spills (bytes stored: N = 27 8, 30 44, 32 120, 36 624).
+// What it replaces: seven launches, and three more for every grid size among the members, each
 // of them short of work (a 27^3 plane keeps 14 lines busy in a block of 1,024 threads) and
-// each a round trip of the grids through L2.  128 boxes of 216 to 2,000 waters: 806 -> 748
-// us a step; bound by its largest member (a block per SM).  One box alone is faster with
-// the launches (648 atoms: 26.3 against 29.4 us a step).
+// each a round trip of the grids through L2.  128 boxes of 216 to 2,000 waters: 806 -> 754
+// us a step; bound by its largest member (a block per SM).  36^3 grids by themselves (boxes of
+// 2,000 to 2,600 waters, us a step, blocks / launches): 8 members 187 / 196, 24 331 / 352, 48
+// 568 / 587.  One box alone is faster with the launches (648 atoms: 26.3 against 29.4).
 constexpr int kBoxThreads = 640;  // 544 lines at N = 32; 96 registers a thread
 #define FZ_BOX_SIZES(X) X(16) X(18) X(20) X(24) X(25) X(27) X(30) X(32) X(36)
 
@@ -1425,8 +1427,15 @@ __global__ void __launch_bounds__(kBoxThreads) k_pme_box_b(const PmeArgs* __rest
   }
 }
 
+// Atoms above which a member keeps the launches.  Spread and gather take a block of 640
+// threads 8 to 13 us per 1,000 atoms, and with a grid coarser than the usual 1.2 A that
+// outgrows what it saves.  us a step of 8 members, blocks / launches: 6,000 atoms on 16^3 142 /
+// 156, on 24^3 120 / 131, on 36^3 132 / 133; 9,000 on 24^3 173 / 154 and 156 / 157 (two runs),
+// on 32^3 180 / 173; 12,000 on 32^3 245 / 199 and 225 / 198.
+constexpr int kBoxAtoms = 8000;
+
 bool pme_box_ok(const PmeArgs& a) {
-  if (a.K[0] != a.K[1] || a.K[0] != a.K[2]) return false;
+  if (a.K[0] != a.K[1] || a.K[0] != a.K[2] || a.n > kBoxAtoms) return false;
   switch (a.K[0]) {
 #define FZ_C(N) case N: return true;
     FZ_BOX_SIZES(FZ_C)

@@ -266,6 +266,8 @@ fz_status fz_batch_free(fz_batch* batch);
 /* Removes a system (it keeps its device state and can be stepped alone or added again). */
 fz_status fz_batch_remove(fz_batch* batch, fz_system* sys);
 fz_status fz_batch_size(fz_batch* batch, int* out);
+/* Kernels that one step of the batch launches (0 before its first step). */
+fz_status fz_batch_launches(fz_batch* batch, long long* out);
 
 /* Serving loop (no counterpart in the reference, which runs one system per process):
  * a worker thread admits submitted jobs in FIFO order while the estimated device
