@@ -440,6 +440,12 @@ static fz_status build_engine(fz_system* s, int device, void* stream) {
     e->nb_per_sm = per;
     e->n_sm = dev_sms;
   }
+  // Four lanes a water up to two blocks per SM (launch_water).  us a step, one lane / four:
+  // 1,000 waters 35.4 / 34.8, 3,000 45.1 / 44.1, 5,360 and 40 chains 65.1 / 63.3, 7,000 67.9 /
+  // 66.7, 9,500 83.2 / 83.4, 11,000 90.6 / 90.6, 12,000 96.4 / 97.4, 15,000 108.6 / 110.5, 28,000
+  // 159.5 / 166.6.  The numbers are the same either way.  FZ_FEW_WATERS: another line.
+  e->few_waters = 64 * dev_sms;
+  if (const char* v = std::getenv("FZ_FEW_WATERS")) e->few_waters = std::max(0, std::atoi(v));
   // ---- atom arrays
   std::vector<float4> pos4(n), vel4(n);
   double mt = 0;

@@ -69,6 +69,7 @@ struct Engine {
   fzk::UnitTerms* unit_terms = nullptr;
   int* unit_term_of = nullptr;
   int unit_term_begin = 0;
+  int few_waters = 0;  // see IntegrateArgs
   float4* pos_drift = nullptr;  // drifted positions of this step, never wrapped by a rebuild
   int* rs_seg = nullptr;
   float* rs_mass = nullptr;
@@ -363,6 +364,7 @@ struct Engine {
     a.unit_term_of = unit_term_of;
     a.unit_term_begin = unit_term_begin;
     a.fuse_terms = unit_terms ? 1 : 0;
+    a.few_waters = few_waters;
     a.vel4 = vel4;
     a.facc = facc;
     a.xyzq_s = xyzq_s;

@@ -998,14 +998,12 @@ static int unit_grid(const IntegrateArgs& a) { return (a.u_end - a.u_begin + 127
 static bool free_and_water(const IntegrateArgs& a) {
   return a.settle && a.ncls == 2 && a.cls_na[0] == 1 && a.cls_nc[0] == 0 && a.cls_na[1] == 3 && a.cls_nc[1] == 3;
 }
-// Lanes per water: one lane each leaves SMs without a block below 148 x 128 waters; four
-// then shorten the pass (bound by one thread's chain) and still fit side by side.
-constexpr int kFewWaters = 148 * 128;
-
+// Lanes per water: one each leaves much of the GPU idle in a small system, whose pass lasts
+// as long as one thread's chain; four shorten it and still fit side by side (a.few_waters).
 template <bool NPT, bool CLOSE>
 static void launch_free_water(const IntegrateArgs& a, cudaStream_t st) {
   const int n = a.cls_begin[2] - a.cls_begin[1], nf = (a.cls_begin[1] - a.cls_begin[0] + 127) / 128;
-  if (n <= kFewWaters)
+  if (n <= a.few_waters)
     launch_pdl(k_drift_free_water<NPT, CLOSE, 4>, dim3((4 * n + 127) / 128 + nf), dim3(128), 0, st, a, (4 * n + 127) / 128);
   else
     launch_pdl(k_drift_free_water<NPT, CLOSE, 1>, dim3((n + 127) / 128 + nf), dim3(128), 0, st, a, (n + 127) / 128);
@@ -1013,7 +1011,7 @@ static void launch_free_water(const IntegrateArgs& a, cudaStream_t st) {
 template <bool NPT, bool CLOSE>
 static void launch_water(const IntegrateArgs& a, cudaStream_t st) {
   const int n = a.u_end - a.u_begin;
-  if (n <= kFewWaters)
+  if (n <= a.few_waters)
     launch_pdl(k_drift_water<NPT, CLOSE, 4>, dim3((4 * n + 127) / 128), dim3(128), 0, st, a);
   else
     launch_pdl(k_drift_water<NPT, CLOSE, 1>, dim3((n + 127) / 128), dim3(128), 0, st, a);

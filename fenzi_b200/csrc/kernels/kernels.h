@@ -201,6 +201,7 @@ struct IntegrateArgs {
   const int* unit_term_of;   // indexed by unit - unit_term_begin
   int unit_term_begin;
   int fuse_terms;
+  int few_waters;           // up to this many SETTLE units take four lanes each (launch_water)
   float4* vel4;             // xyz velocity, w = 1/m
   long long* facc;
   float4* xyzq_s;

@@ -2,8 +2,9 @@
 are integers).  In a step the rigid waters' own terms come from the integrator's pass, and PME
 and the other bonded terms read the positions before a rebuild wraps them; a force call has
 every term from its own kernel and reads the wrapped ones.  Steps that rebuild are among those
-compared.  With chains (two unit classes in one launch) and without; the terms themselves are
-checked against the oracle in test_gpu_terms.py."""
+compared.  With chains (two unit classes in one launch) and without, around the 32 waters of a
+block with four lanes each and the 128 of one with a lane each; the terms themselves are checked
+against the oracle in test_gpu_terms.py."""
 import numpy as np
 import pytest
 
@@ -22,8 +23,10 @@ def _start(nw, chains, T=300.0):
     return s
 
 
-@pytest.mark.parametrize("nw,chains", [(127, 0), (128, 2), (129, 0), (400, 3)])
-def test_forces_left_by_a_step_equal_a_force_call(nw, chains):
+@pytest.mark.parametrize("few", ["0", "1000000"], ids=["one_lane", "four_lanes"])
+@pytest.mark.parametrize("nw,chains", [(127, 0), (128, 2), (129, 0), (160, 1), (161, 0), (400, 3)])
+def test_forces_left_by_a_step_equal_a_force_call(nw, chains, few, monkeypatch):
+    monkeypatch.setenv("FZ_FEW_WATERS", few)
     s = _start(nw, chains)
     at_rebuild = 0
     for n in (1, 2, 3) + (1,) * 20:
@@ -49,4 +52,35 @@ def test_a_run_does_not_depend_on_its_print_interval(nw, chains):
     assert np.array_equal(a.positions(), b.positions())
     assert np.array_equal(a.velocities(), b.velocities())
     for s in (a, b):
+        s.close()
+
+
+@pytest.mark.parametrize("npt", [False, True], ids=["chunk_graph", "barostat"])
+@pytest.mark.parametrize("nw,chains", [(127, 0), (129, 2), (400, 3)])
+def test_one_lane_a_water_equals_four(nw, chains, npt, monkeypatch):
+    """Every form of the pass: alone, beside free atoms, closing the step before, under the
+    barostat."""
+    runs = []
+    for few in ("0", "1000000"):
+        monkeypatch.setenv("FZ_FEW_WATERS", few)
+        s = _start(nw, chains)
+        if npt:
+            s.set_barostat(True, pref_atm=1.0, pmass=1e-5)
+        s.SingleStep(20 if npt else 107)
+        runs.append((s.positions(), s.velocities(), s.forces_fixed()))
+        s.close()
+    for a, b in zip(*runs):
+        assert np.array_equal(a, b)
+
+
+def test_the_line_between_one_lane_and_four(monkeypatch):
+    """A system of as many waters as the line and one of one more: the two sides of the rule."""
+    for few in ("400", "399"):
+        monkeypatch.setenv("FZ_FEW_WATERS", few)
+        s = _start(400, 3)
+        s.SingleStep(25)
+        if few == "400":
+            want = s.positions()
+        else:
+            assert np.array_equal(want, s.positions())
         s.close()
