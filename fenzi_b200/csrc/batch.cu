@@ -181,9 +181,7 @@ static bool batched_kernels_ok(const fz_batch* b) {
   if (v && std::atoi(v) == 0) return false;
   for (const fz_system* s : b->systems) {
     const Engine* e = s->eng;
-    if (e->restraint || e->npt || !fzk::pme_batchable(e->pme_args()) ||
-        !fzk::columns_scan_in_block(e->rebuild_args()))
-      return false;
+    if (e->restraint || e->npt || !fzk::pme_batchable(e->pme_args())) return false;
   }
   return true;
 }
@@ -261,6 +259,7 @@ static fz_status build_batch_kernels(fz_batch* b) {
     if (box) boxes.push_back({pa.K[0], i});
     add_blocks(tabs[fzk::BT_ATOMS256], i, (p.n + 255) / 256);
     add_blocks(tabs[fzk::BT_COLUMNS], i, p.ncol[0] * p.ncol[1]);
+    if (!fzk::columns_scan_in_block(rb.back())) add_blocks(tabs[fzk::BT_SCAN], i, 1);
     add_blocks(tabs[fzk::BT_SLOTS256], i, (p.nslots + 255) / 256);
     add_blocks(tabs[fzk::BT_BLOCKS8], i, (p.nslots / 32 + 7) / 8);
     add_blocks(tabs[fzk::BT_NB], i,
@@ -338,7 +337,7 @@ static fz_status build_batch_kernels(fz_batch* b) {
     FZ_CUDA(cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming));
   }
   if ((r = bk->place(b->arena, b->master))) return r;
-  bk->launches = 2 * (long long)bk->classes.size() + fzk::kRebuildLaunches +
+  bk->launches = 2 * (long long)bk->classes.size() + fzk::kRebuildLaunches + (bk->t.n[fzk::BT_SCAN] > 0 ? 1 : 0) +
                  1 + (bk->t.n[fzk::BT_BONDED] > 0 ? 1 : 0) + (bk->t.n[fzk::BT_BOX] > 0 ? 1 : 0) +
                  (bk->sizes.empty() ? 0 : 7 + 3 * (long long)bk->sizes.size());
   b->bk = std::move(bk);

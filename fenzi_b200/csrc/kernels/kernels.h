@@ -9,7 +9,7 @@ constexpr int kColCap = 4096;  // atoms per column sorted in shared memory
 constexpr int kWarpsPerCta = 8;  // warps of a pair-kernel CTA
 constexpr int kNbBatchCtasPerSm = 4;  // CTAs per SM the batched pair kernel is built and launched for
 // kernels each launcher issues (the step's launch count)
-constexpr int kRebuildLaunches = 6;  // launch_rebuild without its close, launch_rebuild_b
+constexpr int kRebuildLaunches = 6;  // launch_rebuild without its close, launch_rebuild_b (one more if columns are scanned apart)
 
 // Batched launches: one kernel launch covers many systems.  A block table holds one
 // int4 per launched block: (index into the launch's argument array, the block's index
@@ -21,6 +21,7 @@ enum : int {
   BT_BOX,         // one block per system whose PME is done by one block
   BT_ATOMS256,    // (n + 255) / 256
   BT_COLUMNS,     // x-y columns of the neighbour sort
+  BT_SCAN,        // one block per system whose columns are scanned by a launch of its own
   BT_SLOTS256,    // (sorted slots + 255) / 256
   BT_BLOCKS8,     // (32-slot blocks + 7) / 8
   BT_NB,          // pair-kernel CTAs

@@ -71,12 +71,13 @@ __global__ void k_rb_bin_b(const RebuildArgs* __restrict__ args, const int4* __r
 
 
 // exclusive scan of the 32-padded column sizes by one block: start[c] for every column;
-// `publish`: this block also writes what the later launches read
+// `publish`: this block also writes what the later launches read; NT threads
+template <int NT>
 __device__ __forceinline__ void rb_scan(const RebuildArgs& A, int* start, bool publish) {
   const SysParams& p = A.p;
   const int ncol = p.ncol[0] * p.ncol[1];
-  __shared__ int part[256];
-  const int t = threadIdx.x, nt = blockDim.x;
+  __shared__ int part[NT];
+  const int t = threadIdx.x, nt = NT;
   const int per = (ncol + nt - 1) / nt;
   const int b = t * per, e = min(ncol, b + per);
   int s = 0;
@@ -106,10 +107,16 @@ __device__ __forceinline__ void rb_scan(const RebuildArgs& A, int* start, bool p
 }
 
 // systems of more columns than a block scans in shared memory: a launch of its own
-__global__ void __launch_bounds__(256) k_rb_scan(RebuildArgs a) {
+__global__ void __launch_bounds__(1024) k_rb_scan(RebuildArgs a) {
   griddep_wait();
   if (!*a.flag) return;
-  rb_scan(a, a.col_start, true);
+  rb_scan<1024>(a, a.col_start, true);
+}
+__global__ void __launch_bounds__(1024) k_rb_scan_b(const RebuildArgs* __restrict__ args, const int4* __restrict__ tab) {
+  griddep_wait();
+  const RebuildArgs& a = args[tab[blockIdx.x].x];
+  if (!*a.flag) return;
+  rb_scan<1024>(a, a.col_start, true);
 }
 
 // Atoms into their columns.  Every block scans the column sizes itself (a few hundred
@@ -121,7 +128,7 @@ __device__ __forceinline__ void rb_scatter_body(const RebuildArgs& A, int bid, i
   const SysParams& p = A.p;
   if (!*A.flag) return;
   __shared__ int start_s[SCANNED ? 1 : kScanCols];
-  if (!SCANNED) rb_scan(A, start_s, bid == 0);
+  if (!SCANNED) rb_scan<256>(A, start_s, bid == 0);
   const int* start = SCANNED ? A.col_start : start_s;
   const int a = bid * blockDim.x + threadIdx.x;
   if (a >= p.n) return;
@@ -141,7 +148,8 @@ __global__ void __launch_bounds__(256) k_rb_scatter(RebuildArgs a) { griddep_wai
 __global__ void __launch_bounds__(256) k_rb_scatter_b(const RebuildArgs* __restrict__ args, const int4* __restrict__ tab) { griddep_wait();
   const int4 t = tab[blockIdx.x];
   const RebuildArgs a = args[t.x];
-  rb_scatter_body<false>(a, t.y, t.z);
+  if (a.p.ncol[0] * a.p.ncol[1] <= kScanCols) rb_scatter_body<false>(a, t.y, t.z);
+  else rb_scatter_body<true>(a, t.y, t.z);
 }
 
 
@@ -894,7 +902,7 @@ void launch_rebuild(const RebuildArgs& a, cudaStream_t st, bool close) {
   if (columns_scan_in_block(a)) {
     launch_pdl(k_rb_scatter<false>, dim3((p.n + 255) / 256), dim3(256), 0, st, a);
   } else {
-    launch_pdl(k_rb_scan, dim3(1), dim3(256), 0, st, a);
+    launch_pdl(k_rb_scan, dim3(1), dim3(1024), 0, st, a);
     launch_pdl(k_rb_scatter<true>, dim3((p.n + 255) / 256), dim3(256), 0, st, a);
   }
   launch_pdl(k_rb_colsort, dim3(ncol), dim3(256), kColCap * sizeof(unsigned long long), st, a);
@@ -925,17 +933,9 @@ bool prune_split_fits(int ocap) {
 // ------------------------------------------------------------------ batched launchers
 // One launch per kernel over many systems: block b of the launch runs block t.y (of
 // t.z) of system t.x, t = tab[b]; the per-system grids are those of the launchers above.
-void rebuild_grids(const RebuildArgs& a, int* g6) {
-  const SysParams& p = a.p;
-  const int maxblk = p.nslots / 32;
-  g6[0] = (p.n + 255) / 256;          // bin, scatter
-  g6[1] = p.ncol[0] * p.ncol[1];      // colsort
-  g6[2] = (p.nslots + 255) / 256;     // slots
-  g6[3] = (maxblk + 7) / 8;           // outer, prune
-}
-
 void launch_rebuild_b(const RebuildArgs* args, const BatchTables& t, cudaStream_t st) {
   launch_pdl(k_rb_bin_b, dim3(t.n[BT_ATOMS256]), dim3(256), 0, st, args, t.tab[BT_ATOMS256]);
+  if (t.n[BT_SCAN] > 0) launch_pdl(k_rb_scan_b, dim3(t.n[BT_SCAN]), dim3(1024), 0, st, args, t.tab[BT_SCAN]);
   launch_pdl(k_rb_scatter_b, dim3(t.n[BT_ATOMS256]), dim3(256), 0, st, args, t.tab[BT_ATOMS256]);
   launch_pdl(k_rb_colsort_b, dim3(t.n[BT_COLUMNS]), dim3(256), kColCap * sizeof(unsigned long long), st, args, t.tab[BT_COLUMNS]);
   launch_pdl(k_rb_slots_b, dim3(t.n[BT_SLOTS256]), dim3(256), 0, st, args, t.tab[BT_SLOTS256]);

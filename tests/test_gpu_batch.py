@@ -135,3 +135,37 @@ def test_batch_follows_members_of_another_box_or_uploaded_anew(kernels, monkeypa
     b.close()
     for s in alone + mixed + [piston]:
         s.close()
+
+
+def test_members_of_many_columns_take_the_batched_kernels(monkeypatch, tmp_path):
+    """A wide flat box has more sorting columns (here 65 x 65) than a block scans in shared
+    memory; the batch scans that member's by a launch of its own and keeps its kernels for
+    all members, which move as they do alone."""
+    monkeypatch.setenv("FZ_COL_ATOMS", "8")
+    flat = gen_system.build(name="flat", nw=6000, kgrid=64, rc=5.0, ron=4.0, seed=8)
+    own = flat.pos.reshape(-1, 3, 3) - flat.pos.reshape(-1, 3, 3)[:, :1]
+    own -= np.round(own / flat.box) * flat.box
+    flat.box = np.array([1400.0, 1400.0, 11.5])
+    k = np.arange(6000)
+    site = np.stack([(k % 78 + 0.5) / 78 * 1400 - 700, (k // 78 + 0.5) / 78 * 1400 - 700, np.zeros(6000)], 1)
+    flat.pos = (site[:, None] + own).reshape(-1, 3)
+    specs = [gen_system.ensemble(nsys=1, seed=3, nw_min=300, nw_max=300)[0], flat]
+    alone = [_load(s, str(tmp_path / f"a{i}")) for i, s in enumerate(specs)]
+    for s in alone:
+        s.SingleStep(15)
+    launches = {}
+    for mode in ("1", "0"):
+        monkeypatch.setenv("FZ_BATCH_KERNELS", mode)
+        mixed = [_load(s, str(tmp_path / f"b{mode}{i}")) for i, s in enumerate(specs)]
+        b = fz.Batch(mixed)
+        b.step(15)
+        launches[mode] = b.launches_per_step()
+        for a, m in zip(alone, mixed):
+            assert np.array_equal(a.positions(), m.positions())
+            assert np.array_equal(a.forces_fixed(), m.forces_fixed())
+        b.close()
+        for s in mixed:
+            s.close()
+    assert launches["1"] < launches["0"]
+    for s in alone:
+        s.close()
