@@ -489,6 +489,28 @@ struct Engine {
     return (nbond_step + nangle_step + nub + ndihe + nimpr + nexcl_step + n14 > 0) ? 1 : 0;
   }
   int bonded_launches() const { return (nbond + nangle + nub + ndihe + nimpr + nexcl + n14 > 0) ? 1 : 0; }
+  // One pass of the integrator over all unit classes, which touch disjoint atoms: where
+  // they take more than one launch, the first half of them runs on st3 beside the rest.
+  template <class L>
+  void integrate(const fzk::IntegrateArgs& ia, int passes, L launch) {
+    if (passes < 2) return launch(ia, st);
+    const int h = ia.ncls / 2;
+    fzk::IntegrateArgs first = ia, rest = ia;
+    first.ncls = h;
+    rest.ncls = ia.ncls - h;
+    for (int c = 0; c < rest.ncls; ++c) {
+      rest.cls_na[c] = ia.cls_na[c + h];
+      rest.cls_nc[c] = ia.cls_nc[c + h];
+      rest.cls_begin[c] = ia.cls_begin[c + h];
+    }
+    rest.cls_begin[rest.ncls] = ia.cls_begin[ia.ncls];
+    cudaEventRecord(ev_top, st);
+    cudaStreamWaitEvent(st3, ev_top, 0);
+    launch(first, st3);
+    cudaEventRecord(ev_join3, st3);
+    launch(rest, st);
+    cudaStreamWaitEvent(st, ev_join3, 0);
+  }
   // One MD step.  open: the step starts with its own kick + drift pass (else the
   // previous step left its closing kick + RATTLE to this step's first pass); close: the
   // step ends with the kick + RATTLE pass (else the next step's first pass does it).
@@ -510,8 +532,10 @@ struct Engine {
     cudaEventRecord(ev_top, st);
     cudaStreamWaitEvent(st2, ev_top, 0);
     fzk::launch_pme_clear(pa, st2);
-    if (open) fzk::launch_kick_drift(ia, st);
-    else fzk::launch_close_kick_drift(ia, st);
+    integrate(ia, fzk::drift_launches(ia), [&](const fzk::IntegrateArgs& a, cudaStream_t s) {
+      if (open) fzk::launch_kick_drift(a, s);
+      else fzk::launch_close_kick_drift(a, s);
+    });
     cudaEventRecord(ev_fork, st);
     cudaStreamWaitEvent(st2, ev_fork, 0);
     fzk::launch_pme(pa, false, st2, true);
@@ -527,7 +551,10 @@ struct Engine {
     if (bonded) cudaStreamWaitEvent(st, ev_join3, 0);
     cudaEventRecord(ev_join, st2);
     cudaStreamWaitEvent(st, ev_join, 0);
-    if (close) fzk::launch_kick_rattle(ia, false, true, st);
+    if (close)
+      integrate(ia, ia.ncls, [](const fzk::IntegrateArgs& a, cudaStream_t s) {
+        fzk::launch_kick_rattle(a, false, true, s);
+      });
   }
   fz_status graph_step() {
     if (!step_exec) {
