@@ -864,6 +864,7 @@ fz_status set_box(Engine* e, double L) {
   }
   t.beta = (double)p.beta;
   fzk::launch_pme_tables(t, e->st);
+  e->launches += 1;
   FZ_CUDA(cudaGetLastError());
   return FZ_OK;
 }
@@ -960,7 +961,8 @@ static fz_status npt_step(Engine* e) {
   ia = e->int_args();
   ia.vfric = std::exp(-0.5 * dt * e->Ldot / Ln);
   fzk::launch_kick_rattle(ia, false, true, e->st);
-  e->launches += 3 * e->ncls;  // kick/drift, unit virial, kick/RATTLE (forces() counts its own)
+  // kick/drift, unit virial, kick/RATTLE (forces() and set_box() count their own)
+  e->launches += fzk::drift_launches(ia) + 2 * e->ncls;
   return FZ_OK;
 }
 

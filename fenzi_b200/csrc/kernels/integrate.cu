@@ -398,60 +398,57 @@ template <int LPW>
 __device__ __forceinline__ void water_terms(const IntegrateArgs& a, int u, const Unit& U, const float4* x, int q) {
   long long f[3][3] = {};
   const int n = a.p.n;
-  const int t = a.unit_term_of[u - a.unit_term_begin];
-  if (t >= 0) {
-    const UnitTerms T = a.unit_terms[t];
-    const SysParams& p = a.p;
-    const double L[3] = {(double)p.box.x, (double)p.box.y, (double)p.box.z};
-    double d[3][3];  // atoms (0,1), (0,2), (1,2)
+  const UnitTerms T = a.unit_terms[a.unit_term_of[u - a.unit_term_begin]];
+  const SysParams& p = a.p;
+  const double L[3] = {(double)p.box.x, (double)p.box.y, (double)p.box.z};
+  double d[3][3];  // atoms (0,1), (0,2), (1,2)
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const float4 ra = x[k == 2 ? 1 : 0], rb = x[k == 0 ? 1 : 2];
+    d[k][0] = (double)ra.x - (double)rb.x;
+    d[k][1] = (double)ra.y - (double)rb.y;
+    d[k][2] = (double)ra.z - (double)rb.z;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) d[k][c] -= L[c] * rint(d[k][c] * a.inv_box_d[c]);
+  }
+  if constexpr (LPW == 1) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      const float4 ra = x[k == 2 ? 1 : 0], rb = x[k == 0 ? 1 : 2];
-      d[k][0] = (double)ra.x - (double)rb.x;
-      d[k][1] = (double)ra.y - (double)rb.y;
-      d[k][2] = (double)ra.z - (double)rb.z;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) d[k][c] -= L[c] * rint(d[k][c] * a.inv_box_d[c]);
-    }
-    if constexpr (LPW == 1) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const int i = k == 2 ? 1 : 0, j = k == 0 ? 1 : 2;
-        long long g[3];
-        pair_terms(a, T, x, d[k], k, i, j, g);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          f[i][c] += g[c];
-          f[j][c] -= g[c];
-        }
-      }
-      if (T.has >> 3 & 1) apex_terms(T, d[0], d[1], f);
-    } else {
-      const unsigned mask = 0xfu << (threadIdx.x & 28);
-      const int k = min(q, 2);
-      double dk[3];
-      float4 y[2];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) dk[c] = k == 0 ? d[0][c] : (k == 1 ? d[1][c] : d[2][c]);
-      y[0] = k == 2 ? x[1] : x[0];
-      y[1] = k == 0 ? x[1] : x[2];
-      UnitTerms Tk = T;
-      Tk.bond[0] = k == 0 ? T.bond[0] : (k == 1 ? T.bond[1] : T.bond[2]);
-      Tk.has = ((T.has >> k) & 1) | (((T.has >> (5 + k)) & 1) << 5);
-      long long g[3] = {0, 0, 0};
-      if (q < 3) pair_terms(a, Tk, y, dk, 0, 0, 1, g);
-      else if (T.has >> 3 & 1) apex_terms(T, d[0], d[1], f);
-      // atom 0: pairs 0 + 1, atom 1: pair 2 - pair 0, atom 2: - pair 1 - pair 2; and the angle
+      const int i = k == 2 ? 1 : 0, j = k == 0 ? 1 : 2;
+      long long g[3];
+      pair_terms(a, T, x, d[k], k, i, j, g);
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        const long long g0 = __shfl_sync(mask, g[c], 0, 4), g1 = __shfl_sync(mask, g[c], 1, 4),
-                        g2 = __shfl_sync(mask, g[c], 2, 4);
-        const long long a0 = __shfl_sync(mask, f[0][c], 3, 4), a1 = __shfl_sync(mask, f[1][c], 3, 4),
-                        a2 = __shfl_sync(mask, f[2][c], 3, 4);
-        f[0][c] = g0 + g1 + a0;
-        f[1][c] = g2 - g0 + a1;
-        f[2][c] = a2 - g1 - g2;
+        f[i][c] += g[c];
+        f[j][c] -= g[c];
       }
+    }
+    if (T.has >> 3 & 1) apex_terms(T, d[0], d[1], f);
+  } else {
+    const unsigned mask = 0xfu << (threadIdx.x & 28);
+    const int k = min(q, 2);
+    double dk[3];
+    float4 y[2];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) dk[c] = k == 0 ? d[0][c] : (k == 1 ? d[1][c] : d[2][c]);
+    y[0] = k == 2 ? x[1] : x[0];
+    y[1] = k == 0 ? x[1] : x[2];
+    UnitTerms Tk = T;
+    Tk.bond[0] = k == 0 ? T.bond[0] : (k == 1 ? T.bond[1] : T.bond[2]);
+    Tk.has = ((T.has >> k) & 1) | (((T.has >> (5 + k)) & 1) << 5);
+    long long g[3] = {0, 0, 0};
+    if (q < 3) pair_terms(a, Tk, y, dk, 0, 0, 1, g);
+    else if (T.has >> 3 & 1) apex_terms(T, d[0], d[1], f);
+    // atom 0: pairs 0 + 1, atom 1: pair 2 - pair 0, atom 2: - pair 1 - pair 2; and the angle
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const long long g0 = __shfl_sync(mask, g[c], 0, 4), g1 = __shfl_sync(mask, g[c], 1, 4),
+                      g2 = __shfl_sync(mask, g[c], 2, 4);
+      const long long a0 = __shfl_sync(mask, f[0][c], 3, 4), a1 = __shfl_sync(mask, f[1][c], 3, 4),
+                      a2 = __shfl_sync(mask, f[2][c], 3, 4);
+      f[0][c] = g0 + g1 + a0;
+      f[1][c] = g2 - g0 + a1;
+      f[2][c] = a2 - g1 - g2;
     }
   }
 #pragma unroll

@@ -197,7 +197,7 @@ struct IntegrateArgs {
   float4* pos_drift;        // copy of the drifted positions that no rebuild wraps: what PME
                             // and the bonded kernel of a step read
   // terms among the atoms of a SETTLE unit, evaluated where its new positions are made
-  // (fuse_terms; else the bonded kernel has them): term set of each unit, -1 none
+  // (fuse_terms; else the bonded kernel has them): term set of each unit
   const UnitTerms* unit_terms;
   const int* unit_term_of;   // indexed by unit - unit_term_begin
   int unit_term_begin;

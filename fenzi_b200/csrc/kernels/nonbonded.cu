@@ -209,8 +209,9 @@ __device__ __forceinline__ void run_tile(const PairConst& c, const SysParams& p,
   }
 }
 
-// Warp per i-block (blocks taken from a dynamic counter): the diagonal tile, then the
-// block's inner tiles; the i force stays in registers across tiles and is flushed once.
+// A warp per work item, `chunk` tiles of one i-group (the first item by the warp's own number,
+// further ones from a counter): the diagonal tile, then the group's inner tiles; the i forces
+// stay in registers across the item's tiles and are flushed once.
 template <bool ENERGY>
 __device__ __forceinline__ void nonbonded_body(const SysParams& p, const PairConst& c, const float4* __restrict__ xyzq, const int* __restrict__ typ,
     const int* __restrict__ perm, const uint32_t* __restrict__ inner, const int* __restrict__ inner_nt,
