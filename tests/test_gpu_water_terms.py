@@ -14,10 +14,12 @@ from tests.helpers import system
 pytestmark = pytest.mark.gpu
 
 
-def _start(nw, chains, T=300.0):
-    kw = {} if chains == 0 else dict(chain_len=10)
-    _, path = system(f"wt_{nw}_{chains}", name="custom", nw=nw, nchains=chains, rc=6.5, ron=5.0, seed=nw, **kw)
-    s = fz.FenZi.ReadInput(path).LoadSystem()
+def _start(nw, chains, T=300.0, flexible=False):
+    kw = {} if chains == 0 else dict(chain_len=10, extras=flexible)
+    _, path = system(f"wt_{nw}_{chains}_{flexible}", name="custom", nw=nw, nchains=chains, rc=6.5, ron=5.0, seed=nw, **kw)
+    s = fz.FenZi.ReadInput(path)
+    s.cfg.shake = 0 if flexible else 1
+    s.LoadSystem()
     s.InitMem(0)
     s.InitVelocity(T=T, seed=5)
     return s
@@ -41,9 +43,13 @@ def test_forces_left_by_a_step_equal_a_force_call(nw, chains, few, monkeypatch):
     s.close()
 
 
-@pytest.mark.parametrize("nw,chains", [(400, 0), (900, 2)])
-def test_a_run_does_not_depend_on_its_print_interval(nw, chains):
-    a, b = _start(nw, chains), _start(nw, chains)
+@pytest.mark.parametrize("nw,chains,kind", [(400, 0, "rigid"), (900, 2, "rigid"), (900, 2, "flexible"), (900, 2, "barostat")])
+def test_a_run_does_not_depend_on_its_print_interval(nw, chains, kind):
+    """flexible: every bonded term (Urey-Bradley, impropers, two folds) and no constraint."""
+    a, b = (_start(nw, chains, flexible=kind == "flexible") for _ in range(2))
+    if kind == "barostat":
+        for s in (a, b):
+            s.set_barostat(True, pref_atm=1.0, pmass=1e-5)
     for k in range(40):
         a.SingleStep(3)
         b.SingleStep(3)
