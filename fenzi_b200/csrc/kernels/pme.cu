@@ -39,16 +39,22 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
 __device__ __forceinline__ int grid_base(const PmeArgs& a, int d, float x, int K, float* t) {
   const float L = d == 0 ? a.p.box.x : (d == 1 ? a.p.box.y : a.p.box.z);
   const float invL = d == 0 ? a.p.inv_box.x : (d == 1 ? a.p.inv_box.y : a.p.inv_box.z);
-  x = wrap_coord(x, L, invL);
-  const float k = floorf(__fmul_rn(x, a.scale_hi[d]));
-  float f = fmaf(x, a.scale_lo[d], fmaf(x, a.scale_hi[d], -k));
+  const float h = 0.5f * L;
+  float y = x >= h ? x - L : (x < -h ? x + L : x);
+  float k = floorf(__fmul_rn(y, a.scale_hi[d]));
   int k0 = (int)k;
   k0 += k0 < 0 ? K : 0;
-  if (k0 < 0 || k0 >= K) {  // no position of this box (beyond FP32's resolution of it)
-    k0 = 0;
-    f = 0.f;
+  if ((unsigned)k0 >= (unsigned)K) {  // further outside than a period
+    y = wrap_coord(x, L, invL);
+    k = floorf(__fmul_rn(y, a.scale_hi[d]));
+    k0 = (int)k;
+    k0 += k0 < 0 ? K : 0;
+    if ((unsigned)k0 >= (unsigned)K) {  // beyond FP32's resolution of the box
+      k0 = 0;
+      y = k = 0.f;
+    }
   }
-  *t = f;
+  *t = fmaf(y, a.scale_lo[d], fmaf(y, a.scale_hi[d], -k));
   return k0;
 }
 
